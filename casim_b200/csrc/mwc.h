@@ -24,16 +24,22 @@ enum {
     MWC_KO0, MWC_alphakco, MWC_alphakcoI, MWC_kco, MWC_KMgI, MWC_konMgI, MWC_fICa, MWC_fIMg, MWC_gMg, MWC_gCa, MWC_NPAR
 };
 
-// adjacency lists in the reference's order and the stationary distribution of the full
-// Q at the initial mouth values (for InitOpening), built on the host
+// adjacency lists in the reference's order, the transition rates and the stationary
+// distribution of the full Q at the initial mouth values (for InitOpening), built on the
+// host. Every entry of Q is a constant of the parameters times 1, Ca, Mg or Mg^2, so the
+// device multiplies rate[s][k] by the concentration that pick[s][k] names instead of
+// evaluating the entry's powers: 100 sites of 20 RyRs took 440 us a time step with the
+// powers evaluated per RyR and step. Unused slots hold rate 0.
 struct cb_mwc_tab {
     unsigned char nadj[CB_MWC_N];
     unsigned char adj[CB_MWC_N][CB_MWC_MAXADJ];
+    unsigned char pick[CB_MWC_N][CB_MWC_MAXADJ];  // 0: constant, 1: Ca, 2: Mg, 3: Mg^2
+    double rate[CB_MWC_N][CB_MWC_MAXADJ];
     double p_init[CB_MWC_N];
 };
 
 // (i, j, block) of micro-state s, decoded as CaSim/SingleSiteMWC.cpp:156-168 does
-__host__ __device__ inline void cb_mwc_ij(int s, int& i, int& j, int& b) {
+inline void cb_mwc_ij(int s, int& i, int& j, int& b) {
     b = s / 15;
     int r = s - 15 * b;
     for (j = 0; j <= 4; ++j) {
@@ -47,9 +53,9 @@ __host__ __device__ inline void cb_mwc_ij(int s, int& i, int& j, int& b) {
     j = 4;
 }
 
-// Q[s][d] for d adjacent to s, the entries CaSim/SingleSiteMWC.cpp:100-151 (SetRow) sets,
+// host: Q[s][d] for d adjacent to s, the entries CaSim/SingleSiteMWC.cpp:100-151 (SetRow) sets,
 // each with the reference's operand order
-__host__ __device__ inline double cb_mwc_q(const double* P, int s, int d, double ca, double mg) {
+inline double cb_mwc_q(const double* P, int s, int d, double ca, double mg) {
     int i, j, b;
     cb_mwc_ij(s, i, j, b);
     const double fCa4I = P[MWC_fCa4I], fCa = P[MWC_fCa], konCa = P[MWC_konCa], alphaCa = P[MWC_alphaCa];
@@ -98,22 +104,27 @@ __host__ __device__ inline double cb_mwc_q(const double* P, int s, int d, double
     return koc * pow(fIco, 1 - alphakcoI);  // b == 2, db == 1
 }
 
+// Q[s][adj[s][k]] at the mouth concentrations
+__host__ __device__ inline double cb_mwc_rate(const cb_mwc_tab& t, int s, int k, double ca, double mg) {
+    const int p = t.pick[s][k];
+    return t.rate[s][k] * (p == 0 ? 1.0 : p == 1 ? ca : p == 2 ? mg : mg * mg);
+}
+
 // escape rate of s (CaSim/SingleSiteMWC.cpp:162-165)
-__host__ __device__ inline double cb_mwc_exit(const double* P, const cb_mwc_tab& t, int s, double ca, double mg) {
+__host__ __device__ inline double cb_mwc_exit(const cb_mwc_tab& t, int s, double ca, double mg) {
     double r = 0;
-    for (int k = 0; k < t.nadj[s]; ++k) r += cb_mwc_q(P, s, t.adj[s][k], ca, mg);
+#pragma unroll
+    for (int k = 0; k < CB_MWC_MAXADJ; ++k) r += cb_mwc_rate(t, s, k, ca, mg);
     return r;
 }
 
 // destination of a transition out of s for the draw u (CaSim/QMatrixModel.cpp:26-35:
 // the first neighbour whose cumulative rate over the escape rate reaches u; none keeps s)
-__host__ __device__ inline int cb_mwc_next(const double* P, const cb_mwc_tab& t, int s, double ca, double mg, double exit_rate,
-                                           double u) {
+__host__ __device__ inline int cb_mwc_next(const cb_mwc_tab& t, int s, double ca, double mg, double exit_rate, double u) {
     double cum = 0;
     for (int k = 0; k < t.nadj[s]; ++k) {
-        const int d = t.adj[s][k];
-        cum += cb_mwc_q(P, s, d, ca, mg);
-        if (cum / exit_rate >= u) return d;
+        cum += cb_mwc_rate(t, s, k, ca, mg);
+        if (cum / exit_rate >= u) return t.adj[s][k];
     }
     return s;
 }

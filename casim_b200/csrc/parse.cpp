@@ -553,6 +553,12 @@ void cb_mwc_build(const double* P, double ca0, double mg0, cb_mwc_tab& t) {
         for (int k = 0; k < t.nadj[s]; ++k) {
             const int d = t.adj[s][k];
             Q[s][d] = cb_mwc_q(P, s, d, ca0, mg0);
+            // the entry's constant, and the concentration it is proportional to: Ca binding
+            // (+1 within a block), Mg binding (a higher index otherwise), Mg^2 onto the
+            // inhibition site (blocks 0 -> 1 and 3 -> 2), none for the rest
+            t.rate[s][k] = cb_mwc_q(P, s, d, 1.0, 1.0);
+            const int b = s / 15, db = d / 15, del = d - s;
+            t.pick[s][k] = (unsigned char)(b == db ? (del == 1 ? 1 : del > 0 ? 2 : 0) : (b == 0 && db == 1) || (b == 3 && db == 2) ? 3 : 0);
             r += Q[s][d];
         }
         Q[s][s] = -r;

@@ -134,12 +134,12 @@ __global__ void k_pre(cb_model m, int S, int NS, const cb_site* __restrict__ sit
         if (mwc) {
             // SingleSiteMWC: escape rate of the micro-state, the second draw picks where to
             const int mi = ch_micro[st.ch_off + c];
-            const double r = cb_mwc_exit(m.ch_par, *mwc, mi, ca, mg);
+            const double r = cb_mwc_exit(*mwc, mi, ca, mg);
             ++draws;
             if (cbrng::u01d_fold(g) < r * dt) {
                 const double u2 = cbrng::u01d_fold(g);
                 ++draws;
-                const int nx = cb_mwc_next(m.ch_par, *mwc, mi, ca, mg, r, u2);
+                const int nx = cb_mwc_next(*mwc, mi, ca, mg, r, u2);
                 ch_micro[st.ch_off + c] = nx;
                 ch_state[st.ch_off + c] = nx >= CB_MWC_OPEN;
             }
@@ -581,11 +581,12 @@ cudaError_t launch_step(cb_dev& d, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     cudaError_t e0 = mark(0);
     if (e0 != cudaSuccess) return e0;
     const bool fast = stream_tiles(d) > 0;
-    if (fast && !d.mwc && pre_jump(d))
-        stream::k_pre_r<<<(d.S + stream::PRE_WARPS - 1) / stream::PRE_WARPS, 32 * stream::PRE_WARPS, 0, st>>>(
+    if (fast && pre_jump(d)) {
+        auto kern = d.mwc ? stream::k_pre_r<true> : stream::k_pre_r<false>;
+        kern<<<(d.S + stream::PRE_WARPS - 1) / stream::PRE_WARPS, 32 * stream::PRE_WARPS, 0, st>>>(
             d.m, d.S, d.NS, d.sites, d.sc, d.ch_state, d.mouth, d.spx[0], d.spc[0], d.spx[1], d.spc[1], d.pre_jump, d.gates,
-            d.site_gate);
-    else if (d.site_gate)
+            d.site_gate, d.ch_micro, d.mwc);
+    } else if (d.site_gate)
         return cudaErrorNotSupported;  // per-site models need k_pre_r
     else
         k_pre<<<(d.S + 127) / 128, 128, 0, st>>>(d.m, d.S, d.NS, d.sites, d.sc, d.ch_state, d.mouth, d.spx[0], d.spc[0],
