@@ -97,6 +97,13 @@ casim_status set_err(casim_b200_sim* h, casim_status s, const std::string& msg) 
         return set_err(h, CASIM_EINVAL, e.what());                          \
     }
 
+// a kernel's bounded wait for its own copies ran out in an earlier launch (the state is not valid)
+bool wait_gave_up(casim_b200_sim* h) {
+    if (!h->d.err_host || !*(volatile int*)h->d.err_host) return false;
+    h->err = "a kernel's wait for its copies gave up";
+    return true;
+}
+
 void check_site(casim_b200_sim* h, int site) {
     if (site < 0 || site >= h->d.S) throw std::runtime_error("site index " + std::to_string(site) + " out of range");
 }
@@ -131,8 +138,10 @@ void build_device(casim_b200_sim* h, int precision) {
         st.nx = sh.nx;
         st.ny = sh.ny;
         st.nz = cfg.m.dim == 3 ? sh.nz : 1;
-        int N = st.nx * st.ny * st.nz;
-        st.npad = (N + 31) / 32 * 32;
+        st.px = (st.nx + CB_CLEFT_VEC - 1) / CB_CLEFT_VEC * CB_CLEFT_VEC;
+        int N = st.px * st.ny * st.nz;
+        st.npad = (N + 127) / 128 * 128;
+        d.state_nodes += (st.nx * st.ny * st.nz + 31) / 32 * 32;
         st.node_base = nb;
         nb += st.npad;
         st.n_ch = (int)sh.ch_node_xyz.size() / 3;
@@ -146,7 +155,7 @@ void build_device(casim_b200_sim* h, int precision) {
         std::map<int, int> last_at;
         for (int c = 0; c < st.n_ch; ++c) {
             int x = sh.ch_node_xyz[3 * c], y = sh.ch_node_xyz[3 * c + 1], z = sh.ch_node_xyz[3 * c + 2];
-            int node = x + st.nx * (y + st.ny * z);
+            int node = x + st.px * (y + st.ny * z);
             ch_node.push_back(node);
             last_at[node] = c;
         }
@@ -161,7 +170,8 @@ void build_device(casim_b200_sim* h, int precision) {
             for (int r = 0; r < nrim; ++r) {
                 int x, y;
                 cb_rim_xy(r, st.nx, st.ny, x, y);
-                rim_cnode.push_back(cb_rim_cnode(x, y, st.nx, st.ny, cfg.m.dx, cfg.m.dy, cfg.m.hc, mc));
+                const int cn = cb_rim_cnode(x, y, st.nx, st.ny, cfg.m.dx, cfg.m.dy, cfg.m.hc, mc);
+                rim_cnode.push_back(cn % mc + cfg.m.cpx * (cn / mc));
             }
             rimoff += nrim;
             // deposit lists: efflux terms grouped by receiving cytosol node, term order kept
@@ -170,7 +180,8 @@ void build_device(casim_b200_sim* h, int precision) {
                 int x0, y0, x1, y1, x2, y2, z;
                 cb_efflux_term(t, st.nx, st.ny, zmax, x0, y0, x1, y1, x2, y2, z);
                 int r = cb_rim_index(x0, y0, st.nx, st.ny);
-                lists[rim_cnode[st.rim_off + r]].push_back(t);
+                const int cn = rim_cnode[st.rim_off + r];
+                lists[cn % cfg.m.cpx + mc * (cn / cfg.m.cpx)].push_back(t);
             }
             st.term_off = termoff;
             int acc = 0;
@@ -207,7 +218,7 @@ void build_device(casim_b200_sim* h, int precision) {
     for (int k = 0; k < 2; ++k) d.fields[k] = dalloc<char>(h, (size_t)nb * cfg.m.F * rs);
     d.curgrid = dalloc<char>(h, (size_t)nb * cfg.m.n_ions * rs);
     if (rd3d) {
-        d.nc = mc * mc * mc;
+        d.nc = (mc * mc * cfg.m.cpx + 3) / 4 * 4;
         d.CS = cfg.m.n_ions + cfg.m.c_n_pairs;
         for (int k = 0; k < 2; ++k) d.cyto[k] = dalloc<char>(h, (size_t)d.S * d.CS * d.nc * rs);
         d.cin = dalloc<double>(h, (size_t)d.S * d.CS * mc * mc);
@@ -220,8 +231,10 @@ void build_device(casim_b200_sim* h, int precision) {
             d.spx[w] = dupload(h, cfg.sp_x[w]);
             d.spc[w] = dupload(h, cfg.sp_c[w]);
         }
-    d.err_flag = dalloc<int>(h, 4);
-    ck(cudaMemset(d.err_flag, 0, 4 * sizeof(int)), "cudaMemset");
+    // kernels with bounded waits set it; in host memory so that a check costs no copy
+    ck(cudaHostAlloc((void**)&d.err_host, sizeof(int), cudaHostAllocMapped), "cudaHostAlloc");
+    *d.err_host = 0;
+    ck(cudaHostGetDevicePointer((void**)&d.err_flag, d.err_host, 0), "cudaHostGetDevicePointer");
 }
 
 }  // namespace
@@ -269,7 +282,8 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
             // 1024 sites: resident 5.5x and 2.7x the streaming path)
             const bool rd3d = h->d.m.cyto_type == CB_CYTO_RD3D;
             const size_t w = precision == CASIM_FP64 ? 8 : 4;
-            const size_t state = (size_t)h->d.total_nodes * h->d.m.F * w + (rd3d ? (size_t)h->d.S * h->d.CS * h->d.nc * w : 0);
+            const size_t mc = (size_t)h->d.m.mc;
+            const size_t state = (size_t)h->d.state_nodes * h->d.m.F * w + (rd3d ? (size_t)h->d.S * h->d.CS * mc * mc * mc * w : 0);
             int dev = 0, l2 = 0;
             ck(cudaGetDevice(&dev), "cudaGetDevice");
             ck(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev), "cudaDeviceGetAttribute");
@@ -303,6 +317,8 @@ casim_status casim_b200_destroy(casim_h h) {
     if (h->d.rs_counter) cudaFree(h->d.rs_counter);
     if (h->d.rs_pow2) cudaFree(h->d.rs_pow2);
     if (h->d.st_tiles) cudaFree(h->d.st_tiles);
+    if (h->d.st_runs) cudaFree(h->d.st_runs);
+    if (h->d.err_host) cudaFreeHost(h->d.err_host);
     if (h->d.st_chcol) cudaFree(h->d.st_chcol);
     if (h->d.pre_jump) cudaFree(h->d.pre_jump);
     cb_resident_free(h->d);
@@ -335,7 +351,7 @@ casim_status casim_b200_info(casim_h h, casim_info* o) {
     o->n_pairs = h->d.m.n_pairs;
     o->n_buffers = h->d.m.n_buf;
     o->n_cyto_species = h->d.m.n_ions + h->d.m.c_n_pairs;
-    o->cyto_nodes = h->d.nc;
+    o->cyto_nodes = h->d.nc > 0 ? h->d.m.mc * h->d.m.mc * h->d.m.mc : 0;
     o->precision = h->d.precision;
     o->path = h->path;
     o->max_channels = h->d.max_ch;
@@ -443,6 +459,7 @@ casim_status casim_b200_set_site_jsr(casim_h h, const double* jsr) {
 casim_status casim_b200_step(casim_h h, int64_t n) {
     GUARD(h)
     if (n < 0) throw std::runtime_error("negative step count");
+    if (wait_gave_up(h)) return CASIM_ETIMEOUT;
     long long launches = 0;
     ck(cudaEventRecord(h->ev0, h->stream), "cudaEventRecord");
     auto run = [&](long long k) {
@@ -666,6 +683,7 @@ casim_status casim_b200_autotune(casim_h h, int64_t steps_per_trial, char* repor
 casim_status casim_b200_synchronize(casim_h h) {
     GUARD(h)
     ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    if (wait_gave_up(h)) return CASIM_ETIMEOUT;
     float ms = 0;
     // only after a step recorded both events; a failed query must not leave
     // its error behind for the next cudaGetLastError of another library
@@ -715,7 +733,7 @@ casim_status casim_b200_get_field(casim_h h, int32_t site, int32_t species, doub
     for (int z = 0; z < st.nz; ++z)
         for (int y = 0; y < st.ny; ++y)
             for (int x = 0; x < st.nx; ++x) {
-                int n = x + st.nx * (y + st.ny * z);
+                int n = x + st.px * (y + st.ny * z);
                 double v;
                 if (species < m.F) {
                     v = blk[(size_t)species * st.npad + n];
@@ -744,7 +762,7 @@ casim_status casim_b200_set_field(casim_h h, int32_t site, int32_t species, cons
     for (int z = 0; z < st.nz; ++z)
         for (int y = 0; y < st.ny; ++y)
             for (int x = 0; x < st.nx; ++x) {
-                int n = x + st.nx * (y + st.ny * z);
+                int n = x + st.px * (y + st.ny * z);
                 double v = in[ref_index(st, m.dim, x, y, z)];
                 if (rs == 8) ((double*)raw.data())[n] = v;
                 else ((float*)raw.data())[n] = (float)v;
@@ -1050,7 +1068,12 @@ casim_status casim_b200_get_cyto_field(casim_h h, int32_t site, int32_t species,
     std::vector<char> raw((size_t)h->d.nc * rs);
     const char* base = (const char*)h->d.cyto[h->d.ccur] + ((size_t)site * h->d.CS + species) * h->d.nc * rs;
     ck(cudaMemcpy(raw.data(), base, raw.size(), cudaMemcpyDeviceToHost), "cudaMemcpy");
-    for (int n = 0; n < h->d.nc; ++n) out[n] = rs == 8 ? ((double*)raw.data())[n] : (double)((float*)raw.data())[n];
+    const int mc = h->d.m.mc, cpx = h->d.m.cpx;
+    for (int r = 0; r < mc * mc; ++r)
+        for (int i = 0; i < mc; ++i) {
+            const int n = r * cpx + i;
+            out[r * mc + i] = rs == 8 ? ((double*)raw.data())[n] : (double)((float*)raw.data())[n];
+        }
     return CASIM_OK;
     END_GUARD(h)
 }
@@ -1063,10 +1086,14 @@ casim_status casim_b200_set_cyto_field(casim_h h, int32_t site, int32_t species,
     ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
     size_t rs = h->d.precision == 0 ? 8 : 4;
     std::vector<char> raw((size_t)h->d.nc * rs);
-    for (int n = 0; n < h->d.nc; ++n) {
-        if (rs == 8) ((double*)raw.data())[n] = in[n];
-        else ((float*)raw.data())[n] = (float)in[n];
-    }
+    const int mc = h->d.m.mc, cpx = h->d.m.cpx;
+    for (int r = 0; r < mc * mc; ++r)
+        for (int i = 0; i < cpx; ++i) {
+            const int n = r * cpx + i;
+            const double v = in[r * mc + std::min(i, mc - 1)];  // the padding takes the last node's value
+            if (rs == 8) ((double*)raw.data())[n] = v;
+            else ((float*)raw.data())[n] = (float)v;
+        }
     char* base = (char*)h->d.cyto[h->d.ccur] + ((size_t)site * h->d.CS + species) * h->d.nc * rs;
     ck(cudaMemcpy(base, raw.data(), raw.size(), cudaMemcpyHostToDevice), "cudaMemcpy H2D");
     return CASIM_OK;

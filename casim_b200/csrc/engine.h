@@ -19,6 +19,7 @@ struct cb_dev {
     int max_ch = 0;
     int max_terms = 0;      // largest efflux term count of a site
     long long total_nodes = 0;  // sum of npad
+    long long state_nodes = 0;  // sum of nx*ny*nz rounded up to a multiple of 32
     long long total_ch = 0;
     cb_site* sites = nullptr;         // [S]
     cb_site_scalars* sc = nullptr;    // [S]
@@ -32,31 +33,36 @@ struct cb_dev {
     const struct cb_mwc_tab* mwc = nullptr;  // SingleSiteMWC: adjacency and initial distribution
     double* mouth = nullptr;          // [(ch)*NS + species]
     // RD3D cytosol
-    int nc = 0;                       // nodes per site cytosol (mc^3)
+    int nc = 0;                       // stored nodes per site cytosol (mc^2 rows of pitch cpx)
     int CS = 0;                       // cytosol species: ions + cytosol pairs
     void* cyto[2] = {nullptr, nullptr};  // ping-pong, [site][species][node]
     int ccur = 0;
     double* cin = nullptr;            // efflux deposit into layer 0, [site][species][mc*mc]
-    int* rim_cnode = nullptr;         // cytosol layer-0 node (i + mc*j) per rim entry
+    int* rim_cnode = nullptr;         // cytosol layer-0 node (i + cpx*j) per rim entry
     int* dep_ptr = nullptr;           // per site (mc*mc + 1) CSR offsets into dep_term
     int* dep_term = nullptr;          // efflux term indices, oracle order
     // spline tables
     double* spx[2] = {nullptr, nullptr};
     double* spc[2] = {nullptr, nullptr};
     // bookkeeping
-    int* err_flag = nullptr;          // device-side error word
+    int* err_host = nullptr;          // set to 1 by a kernel whose bounded wait ran out (mapped host memory)
+    int* err_flag = nullptr;          // its device address
     // resident path: work queue (sites by decreasing size), its counter and
     // the MRG32k3a jump table A^(2^k), k < 64; allocated on first use
     int* rs_order = nullptr;
     int* rs_counter = nullptr;
     unsigned long long* rs_pow2 = nullptr;
     struct cb_rs_plan* rs_plan = nullptr;  // host-side launch plan (resident.cu)
-    // plain path, specialised stencils: (site, first column) of every cleft block;
+    // plain path, specialised stencils: (site, first group, division by the row pitch) of every cleft block;
     // st_nz = the cleft layers every site shares (0: mixed), -1 before the first step
-    int2* st_tiles = nullptr;
+    int4* st_tiles = nullptr;
     int st_ntiles = 0;
+    void* st_runs = nullptr;  // the tiles of the asynchronous cleft kernel (stream::rd_tile), if it serves the batch
+    int st_nruns = 0, st_grid = 0;
+    bool st_cyt_ready = false;  // the asynchronous cytosol kernel's attributes are set
+    int st_stage[32];         // its shared-memory carve (stream::rd_stage)
     int st_nz = -1;
-    unsigned* st_chcol = nullptr;  // bit per cleft column (node_base + x + nx*y): holds a RyR
+    unsigned* st_chcol = nullptr;  // bit per cleft column (node_base + x + px*y): holds a RyR
     // per-site gating models (plain path): gates[0] the batch's own, site_gate[s] the index
     cb_gate* gates = nullptr;
     int* site_gate = nullptr;

@@ -64,6 +64,7 @@ struct cb_model {
     int c_serca[CB_MAX_IONS];
     double c_Jmax[CB_MAX_IONS], c_Kup[CB_MAX_IONS];
     int mc;     // RD3D nodes per edge
+    int cpx;    // RD3D stored row pitch: mc rounded up to whole CB_CYTO_VEC nodes
     double hc;  // RD3D spacing, nm
     // derived
     double grad_mult;  // 3/(4 pi R^3)
@@ -91,13 +92,18 @@ struct cb_site_scalars {
     int pad;
 };
 
+// Rows of the stored grids are padded to whole groups of nodes that a thread of the
+// streaming stencils loads and stores as one word (2 or 4 floats, 2 doubles).
+constexpr int CB_CLEFT_VEC = 4, CB_CYTO_VEC = 2;
+
 // Packed site table entry (device resident, read-only during stepping).
-// Fields of site s: species f, node n (x fastest: n = x + nx*(y + ny*z)) at
+// Fields of site s: species f, node n (x fastest: n = x + px*(y + ny*z), px = nx rounded up
+// to whole CB_CLEFT_VEC nodes; the padding holds finite values of no meaning) at
 // fields[node_base*F + f*npad + n]; RyR currents at cur[node_base*n_ions + j*npad + n].
 struct cb_site {
-    int nx, ny, nz;
+    int nx, ny, nz, px;
     int n_ch;
-    int npad;              // node count rounded up to a multiple of 32
+    int npad;              // px*ny*nz rounded up to a multiple of 32
     int ch_off;            // first RyR of the site in the channel arrays
     long long node_base;   // sum of npad over the preceding sites
     int rim_off;           // RD3D: first rim entry of the site (rim -> cytosol node table)

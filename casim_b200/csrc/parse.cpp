@@ -432,6 +432,7 @@ cb_config cb_parse_config(const std::string& json_text, const std::string& base_
     if (m.cyto_type == CB_CYTO_RD3D) {
         m.mc = (int)num(c, "Nodes", "Cytosol");
         m.hc = num(c, "dx", "Cytosol");
+        m.cpx = (m.mc + CB_CYTO_VEC - 1) / CB_CYTO_VEC * CB_CYTO_VEC;
         if (m.mc < 4 || m.mc > 64) fail("Cytosol.Nodes must be in [4, 64]");
         if (!(m.hc > 0)) fail("Cytosol.dx must be positive");
         m.inv_hc2 = 1.0 / (m.hc * m.hc);

@@ -164,9 +164,9 @@ __global__ void __launch_bounds__(256) k_cyto(cb_model m, int nc, const R* __res
     const int s = blockIdx.y;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= nc) return;
-    const int mc = m.mc, mc2 = mc * mc;
-    const int i = n % mc, j = (n / mc) % mc, k = n / mc2;
-    if (i == 0 || i == mc - 1 || j == 0 || j == mc - 1 || k == mc - 1) return;
+    const int mc = m.mc, px = m.cpx, mc2 = mc * px;  // mc2: a stored plane
+    const int i = n % px, j = (n / px) % mc, k = n / mc2;
+    if (i == 0 || i >= mc - 1 || j == 0 || j == mc - 1 || k == mc - 1) return;
     const int CS = m.n_ions + m.c_n_pairs;
     const R* u = in + (long long)s * CS * nc;
     R* o = out + (long long)s * CS * nc;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) k_cyto(cb_model m, int nc, const R* __res
         const R* v = u + (long long)c * nc;
         R D = (R)(c < m.n_ions ? m.D_ion[c] : m.c_D_pair[c - m.n_ions]);
         R cc = v[n];
-        evo[c] = D * ((v[n + 1] - 2 * cc + v[n - 1]) * ih2 + (v[n + mc] - 2 * cc + v[n - mc]) * ih2 + (v[zr] - 2 * cc + v[zl]) * ih2);
+        evo[c] = D * ((v[n + 1] - 2 * cc + v[n - 1]) * ih2 + (v[n + px] - 2 * cc + v[n - px]) * ih2 + (v[zr] - 2 * cc + v[zl]) * ih2);
     }
     R fr[CB_MAX_CBUF];
     for (int b = 0; b < m.c_n_buf; ++b) fr[b] = (R)m.c_Ctot[b];
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) k_cyto(cb_model m, int nc, const R* __res
     const R dt = (R)m.dt;
     for (int c = 0; c < CS; ++c) {
         R e = evo[c];
-        if (k == 0) e += (R)cin[((long long)s * CS + c) * mc2 + n];
+        if (k == 0) e += (R)cin[((long long)s * CS + c) * mc * mc + i + mc * j];
         o[(long long)c * nc + n] = u[(long long)c * nc + n] + e * dt;
     }
 }
@@ -216,13 +216,13 @@ __global__ void __launch_bounds__(256) k_rd(cb_model m, const cb_site* __restric
     const int s = blockIdx.y;
     const cb_site st = sites[s];
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nxy = st.nx * st.ny;
+    const int nxy = st.px * st.ny;
     if (n >= nxy * st.nz) return;
     const int F = m.F;
     const R* u = in + st.node_base * F;
     R* o = out + st.node_base * F;
-    const int x = n % st.nx, y = (n / st.nx) % st.ny, z = n / nxy;
-    if (x == 0 || x == st.nx - 1 || y == 0 || y == st.ny - 1) {
+    const int x = n % st.px, y = (n / st.px) % st.ny, z = n / nxy;
+    if (x == 0 || x >= st.nx - 1 || y == 0 || y == st.ny - 1) {
         for (int f = 0; f < F; ++f) o[(long long)f * st.npad + n] = u[(long long)f * st.npad + n];
         return;
     }
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256) k_rd(cb_model m, const cb_site* __restric
         val[f] = c;
         R D = (R)(f < m.n_ions ? m.D_ion[f] : m.D_pair[f - m.n_ions]);
         if (D != (R)0) {
-            R lap = (v[n + 1] - 2 * c + v[n - 1]) * idx2 + (v[n + st.nx] - 2 * c + v[n - st.nx]) * idy2;
+            R lap = (v[n + 1] - 2 * c + v[n - 1]) * idx2 + (v[n + st.px] - 2 * c + v[n - st.px]) * idy2;
             if (m.dim == 3) lap = lap + (v[zr] - 2 * c + v[zl]) * idz2;
             evo[f] = D * lap;
         } else {
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(256) k_update(cb_model m, int NS, const cb_sit
     cb_site_scalars& q = sc[s];
     const int F = m.F;
     R* u = fld + st.node_base * F;
-    const int nx = st.nx, ny = st.ny, nz = st.nz, nxy = nx * ny;
+    const int nx = st.nx, ny = st.ny, nz = st.nz, px = st.px, nxy = px * ny;
     const long long np = st.npad;
     // 1. mouth values: ions, pairs, free buffers (CaSim/DyadRD2DCPU.cpp:361-380)
     for (int c = threadIdx.x; c < st.n_ch; c += blockDim.x) {
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(256) k_update(cb_model m, int NS, const cb_sit
     for (int t = threadIdx.x; t < nrim * nz; t += blockDim.x) {
         int r = t % nrim, z = t / nrim, x, y;
         cb_rim_xy(r, nx, ny, x, y);
-        int node = x + nx * y + nxy * z;
+        int node = x + px * y + nxy * z;
         if (m.cyto_type == CB_CYTO_POOL) {
             for (int j = 0; j < m.n_ions; ++j) u[j * np + node] = (R)q.c_ions[j];
             for (int p = 0; p < m.n_pairs; ++p) u[(m.n_ions + p) * np + node] = (R)q.c_bnd[p];
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(256) k_update(cb_model m, int NS, const cb_sit
         int x0, y0, x1, y1, x2, y2, z;
         int sel = cb_efflux_term(t, nx, ny, zmax, x0, y0, x1, y1, x2, y2, z);
         double sf = sel == 0 ? m.sx : m.sy;
-        int n0 = x0 + nx * y0 + nxy * z, n1 = x1 + nx * y1 + nxy * z, n2 = x2 + nx * y2 + nxy * z;
+        int n0 = x0 + px * y0 + nxy * z, n1 = x1 + px * y1 + nxy * z, n2 = x2 + px * y2 + nxy * z;
         for (int f = 0; f < F; ++f) {
             double D = f < m.n_ions ? m.D_ion[f] : m.D_pair[f - m.n_ions];
             double g = 2 * (double)u[f * np + n1] - 1.5 * (double)u[f * np + n0] - 0.5 * (double)u[f * np + n2];
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(256) k_update(cb_model m, int NS, const cb_sit
 
 // The specialised stencils (stream_kernels.cuh) serve 1-2 ions with up to 4 pairs
 // and a cleft of one layer (2D) or three (3D) at every site; the first step lists
-// the cleft blocks (site, first column). Returns the tile count, 0 if not covered.
+// the cleft blocks (site, first group). Returns the tile count, 0 if not covered.
 int stream_tiles(cb_dev& d) {
     if (d.st_nz >= 0) return d.st_nz > 0 ? d.st_ntiles : 0;
     d.st_nz = 0;
@@ -420,31 +420,88 @@ int stream_tiles(cb_dev& d) {
     std::vector<cb_site> hs(d.S);
     if (cudaMemcpy(hs.data(), d.sites, sizeof(cb_site) * d.S, cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
     const int nz = d.m.dim == 2 ? 1 : 3;
-    std::vector<int2> tiles;
+    const int V = stream::rd_vec(d.precision == 0 ? 8 : 4);
+    std::vector<int4> tiles;
+    std::vector<stream::rd_tile> runs;
+    const int tn = stream::rdt_threads(d.precision == 0 ? 8 : 4) * V;
+    int px_min = INT32_MAX, px_max = 0;
+    bool two_rims = false;  // a tile may hold a site's first and last row
     for (int s = 0; s < d.S; ++s) {
-        if (hs[s].nz != nz) return 0;
-        const int cols = hs[s].nx * hs[s].ny;
-        for (int c = 0; c < cols; c += stream::RD_THREADS) tiles.push_back(make_int2(s, c));
+        if (hs[s].nz != nz || (long long)hs[s].npad * d.m.F > INT32_MAX) return 0;
+        // the row of a column by a multiply and a shift: floor(2^32 (2^w - px) / px) + 1, w =
+        // ceil(log2 px), exact below 2^31 (Granlund and Montgomery 1994)
+        unsigned w = 0;
+        while ((1u << w) < (unsigned)hs[s].px) ++w;
+        const unsigned mul = (unsigned)(((1ull << 32) * ((1ull << w) - hs[s].px)) / hs[s].px + 1);
+        const int groups = hs[s].px * hs[s].ny / V;
+        for (int c = 0; c < groups; c += stream::RD_THREADS) tiles.push_back(make_int4(s, c, (int)mul, (int)w));
+        for (int c = 0; c < groups * V; c += tn) {
+            stream::rd_tile t{};
+            t.node_base = hs[s].node_base;
+            t.site = s;
+            t.col0 = c;
+            t.np = hs[s].npad;
+            t.px = hs[s].px;
+            t.nx = hs[s].nx;
+            t.ny = hs[s].ny;
+            t.rim_off = hs[s].rim_off;
+            t.mul = mul;
+            t.sh = w;
+            runs.push_back(t);
+        }
+        px_min = std::min(px_min, hs[s].px);
+        px_max = std::max(px_max, hs[s].px);
+        two_rims = two_rims || hs[s].px * (hs[s].ny - 2) <= tn;
     }
     if (tiles.empty() || tiles.size() > (size_t)INT32_MAX) return 0;
-    if (cudaMalloc(&d.st_tiles, sizeof(int2) * tiles.size()) != cudaSuccess) return 0;
-    if (cudaMemcpy(d.st_tiles, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (cudaMalloc(&d.st_tiles, sizeof(int4) * tiles.size()) != cudaSuccess) return 0;
+    if (cudaMemcpy(d.st_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaFree(d.st_tiles);
         d.st_tiles = nullptr;
         return 0;
     }
     d.st_ntiles = (int)tiles.size();
-    // the columns that hold a RyR: bit (node_base + x + nx*y), one word per 32 nodes
-    std::vector<unsigned> bits((size_t)(d.total_nodes + 31) / 32, 0u);
+    // the columns that hold a RyR: bit (node_base + x + px*y), one word per 32 nodes
+    // (the last tile of a site may read up to a tile's bits past the end)
+    std::vector<unsigned> bits((size_t)(d.total_nodes + 31) / 32 + 64, 0u);
     std::vector<int> chn((size_t)d.total_ch);
     if (d.total_ch && cudaMemcpy(chn.data(), d.ch_node, sizeof(int) * chn.size(), cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
     for (int s = 0; s < d.S; ++s)
         for (int c = 0; c < hs[s].n_ch; ++c) {
-            const long long b = hs[s].node_base + chn[hs[s].ch_off + c] % (hs[s].nx * hs[s].ny);
+            const long long b = hs[s].node_base + chn[hs[s].ch_off + c] % (hs[s].px * hs[s].ny);
             bits[b >> 5] |= 1u << (b & 31);
         }
     if (cudaMalloc(&d.st_chcol, sizeof(unsigned) * bits.size()) != cudaSuccess) return 0;
     if (cudaMemcpy(d.st_chcol, bits.data(), sizeof(unsigned) * bits.size(), cudaMemcpyHostToDevice) != cudaSuccess) return 0;
+    // shared-memory carve of the asynchronous kernel's stages. It is used where at least two
+    // blocks (FP64) or three (FP32) fit an SM, 12 computing warps; with fewer it is no faster than
+    // k_rd_v (2048 sites, FP32: three blocks 189 us, two 270, k_rd_v 262)
+    {
+        const int rsz = d.precision == 0 ? 8 : 4;
+        stream::rd_stage g{};
+        auto up = [](int v) { return (v + 127) / 128 * 128; };
+        int off = sizeof(stream::rd_tile);
+        g.bits = off;
+        off = up(off + tn / 8);
+        g.rim = off;
+        off = up(off + (2 * (tn / px_min + 2) + (two_rims ? 2 : 1) * px_max) * d.m.F * rsz);
+        g.halo = px_max + 16 / rsz;
+        for (int f = 0; f < d.m.F; ++f) {
+            const bool diff = (f < d.m.n_ions ? d.m.D_ion[f] : d.m.D_pair[f - d.m.n_ions]) != 0;
+            g.plane[f] = off;
+            g.stride[f] = up((tn + (diff ? 2 * g.halo : 0)) * rsz);
+            off += g.stride[f] * nz;
+        }
+        g.bytes = off;
+        const long long block = (long long)off * stream::RDT_STAGES + 2048;
+        if (block * (rsz == 4 ? 3 : 2) <= 228 * 1024) {
+            if (cudaMalloc(&d.st_runs, sizeof(stream::rd_tile) * runs.size()) != cudaSuccess) return 0;
+            if (cudaMemcpy(d.st_runs, runs.data(), sizeof(stream::rd_tile) * runs.size(), cudaMemcpyHostToDevice) != cudaSuccess) return 0;
+            d.st_nruns = (int)runs.size();
+            static_assert(sizeof(g) <= sizeof(d.st_stage), "carve");
+            std::memcpy(d.st_stage, &g, sizeof(g));
+        }
+    }
     d.st_nz = nz;
     return d.st_ntiles;
 }
@@ -504,7 +561,7 @@ cudaError_t launch_update_np(cb_dev& d, cudaStream_t st, bool after_step) {
     }
 }
 
-// after_step: right after k_rd_s, which set the rim already
+// after_step: right after k_rd_v, which set the rim already
 template <typename R>
 cudaError_t launch_update(cb_dev& d, cudaStream_t st, bool after_step = false) {
     if (stream_tiles(d) > 0) {
@@ -526,50 +583,149 @@ cudaError_t launch_update(cb_dev& d, cudaStream_t st, bool after_step = false) {
     return cudaGetLastError();
 }
 
+// constants of the cleft stencil
+template <typename R>
+stream::rd_const<R> rd_constants(const cb_dev& d) {
+    const cb_model& m = d.m;
+    stream::rd_const<R> k{};
+    for (int f = 0; f < m.F; ++f) {
+        const double D = f < m.n_ions ? m.D_ion[f] : m.D_pair[f - m.n_ions];
+        k.ax[f] = stream::both((R)(D * m.dt * m.inv_dx2));
+        k.ay[f] = stream::both((R)(D * m.dt * m.inv_dy2));
+        k.az[f] = stream::both((R)(D * m.dt * m.inv_dz2));
+        k.diff[f] = D != 0;
+        const int cq = f < m.n_ions ? f : m.dyad_c_pair[f - m.n_ions];
+        k.src[f] = f < m.n_ions ? f : cq >= 0 ? m.n_ions + cq : -1;
+        k.init[f] = (R)(f < m.n_ions ? m.Cb[f] : m.pair_init[f - m.n_ions]);
+    }
+    for (int p = 0; p < m.n_pairs; ++p) {
+        k.mkon[p] = stream::both((R)(-m.kon[p] * m.dt));
+        k.koff[p] = stream::both((R)(m.koff[p] * m.dt));
+        k.ctot[p] = stream::both((R)m.Ctot[m.pair_buf[p]]);
+        k.pion[p] = m.pair_ion[p];
+        for (int q = 0; q < m.n_pairs; ++q)
+            if (m.pair_buf[q] == m.pair_buf[p]) k.same[p] |= 1u << q;
+    }
+    for (int j = 0; j < m.n_ions; ++j) {
+        k.has_sl[j] = m.has_sl[j];
+        k.K1[j] = (R)m.K1[j];
+        k.K2[j] = (R)m.K2[j];
+        k.A1[j] = (R)(m.N1[j] * m.K1[j]);
+        k.A2[j] = (R)(m.N2[j] * m.K2[j]);
+    }
+    k.dt = stream::both((R)m.dt);
+    k.CS = d.CS;
+    k.nc = d.nc;
+    return k;
+}
+
+// constants of the RD3D cytosol stencil
+template <typename R>
+stream::cy_const<R> cy_constants(const cb_dev& d) {
+    const cb_model& m = d.m;
+    stream::cy_const<R> k{};
+    for (int c = 0; c < d.CS; ++c) k.a[c] = stream::both((R)((c < m.n_ions ? m.D_ion[c] : m.c_D_pair[c - m.n_ions]) * m.dt * m.inv_hc2));
+    for (int p = 0; p < m.c_n_pairs; ++p) {
+        k.mkon[p] = stream::both((R)(-m.c_kon[p] * m.dt));
+        k.koff[p] = stream::both((R)(m.c_koff[p] * m.dt));
+        k.ctot[p] = stream::both((R)m.c_Ctot[m.c_pair_buf[p]]);
+        k.pion[p] = m.c_pair_ion[p];
+        for (int q = 0; q < m.c_n_pairs; ++q)
+            if (m.c_pair_buf[q] == m.c_pair_buf[p]) k.same[p] |= 1u << q;
+    }
+    int is = 0;
+    for (int j = 0; j < m.n_ions; ++j)
+        if ((k.serca[j] = m.c_serca[j]) != 0) {
+            const double K2 = m.c_Kup[is] * m.c_Kup[is], b2 = m.c_bg[is] * m.c_bg[is];
+            k.mjmax[j] = stream::both((R)(-m.c_Jmax[is] * m.dt));
+            k.k2[j] = stream::both((R)K2);
+            k.mrest[j] = stream::both((R)(-(b2 / (b2 + K2))));
+            ++is;
+        }
+    k.dt = (R)m.dt;
+    k.mc = m.mc;
+    k.px = m.cpx;
+    k.nplane = m.mc * m.cpx;
+    k.nc = d.nc;
+    return k;
+}
+
 template <typename R, int NI, int NP>
-void launch_rd_s(cb_dev& d, cudaStream_t st) {
+cudaError_t launch_rd_s(cb_dev& d, cudaStream_t st) {
+    constexpr int V = stream::rd_vec(sizeof(R));
     const R* in = (const R*)d.fields[d.cur];
     R* out = (R*)d.fields[1 - d.cur];
     // the cytosol as it was before its latest step (k_cyto flipped ccur already)
     const R* cy = (const R*)d.cyto[1 - d.ccur];
-    if (d.st_nz == 1)
-        stream::k_rd_s<R, NI, NP, 1><<<d.st_ntiles, stream::RD_THREADS, 0, st>>>(d.m, d.sites, d.st_tiles, in, out, (const R*)d.curgrid,
-                                                                                 d.sc, cy, d.st_chcol);
-    else
-        stream::k_rd_s<R, NI, NP, 3><<<d.st_ntiles, stream::RD_THREADS, 0, st>>>(d.m, d.sites, d.st_tiles, in, out, (const R*)d.curgrid,
-                                                                                 d.sc, cy, d.st_chcol);
+    if (d.st_runs) {
+        stream::rd_stage g;
+        std::memcpy(&g, d.st_stage, sizeof(g));
+        const int smem = g.bytes * stream::RDT_STAGES;
+        auto kern = d.st_nz == 1 ? stream::k_rd_t<R, NI, NP, 1, V, stream::RDT_STAGES> : stream::k_rd_t<R, NI, NP, 3, V, stream::RDT_STAGES>;
+        cudaError_t e;
+        if (d.st_grid == 0) {
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+            int dev = 0, sms = 0, per = 0;
+            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, stream::rdt_threads(sizeof(R)) + 32, smem)) != cudaSuccess) return e;
+            d.st_grid = std::max(1, std::min(sms * per, d.st_nruns));
+        }
+        kern<<<d.st_grid, stream::rdt_threads(sizeof(R)) + 32, smem, st>>>(rd_constants<R>(d), g, (const stream::rd_tile*)d.st_runs, d.st_nruns, in,
+                                                                          out, (const R*)d.curgrid, d.sc, cy, d.rim_cnode, d.st_chcol, d.err_flag);
+        return cudaGetLastError();
+    }
+    auto kern = d.st_nz == 1 ? stream::k_rd_v<R, NI, NP, 1, V> : stream::k_rd_v<R, NI, NP, 3, V>;
+    kern<<<d.st_ntiles, stream::RD_THREADS, 0, st>>>(rd_constants<R>(d), d.sites, d.st_tiles, in, out, (const R*)d.curgrid, d.sc, cy,
+                                                     d.rim_cnode, d.st_chcol);
+    return cudaGetLastError();
 }
 
 template <typename R, int NI>
-void launch_rd_np(cb_dev& d, cudaStream_t st) {
+cudaError_t launch_rd_np(cb_dev& d, cudaStream_t st) {
     switch (d.m.n_pairs) {
-    case 0: launch_rd_s<R, NI, 0>(d, st); break;
-    case 1: launch_rd_s<R, NI, 1>(d, st); break;
-    case 2: launch_rd_s<R, NI, 2>(d, st); break;
-    case 3: launch_rd_s<R, NI, 3>(d, st); break;
-    default: launch_rd_s<R, NI, 4>(d, st); break;
+    case 0: return launch_rd_s<R, NI, 0>(d, st);
+    case 1: return launch_rd_s<R, NI, 1>(d, st);
+    case 2: return launch_rd_s<R, NI, 2>(d, st);
+    case 3: return launch_rd_s<R, NI, 3>(d, st);
+    default: return launch_rd_s<R, NI, 4>(d, st);
     }
 }
 
 template <typename R, int NI, int NCP>
-void launch_cyto_s(cb_dev& d, cudaStream_t st) {
+cudaError_t launch_cyto_s(cb_dev& d, cudaStream_t st) {
+    constexpr int V = CB_CYTO_VEC;
+    const R* in = (const R*)d.cyto[d.ccur];
+    R* out = (R*)d.cyto[1 - d.ccur];
+    const int planes = d.m.mc - 1;
     if (d.m.mc == 25) {
-        stream::k_cyto_m<R, NI, NCP, 25><<<d.S, 640, 0, st>>>(d.m, (const R*)d.cyto[d.ccur], (R*)d.cyto[1 - d.ccur], d.cin);
-        return;
+        // the planes of a site in 1, 2 or 3 chunks (each but the first loads a plane or two
+        // more) so that a small batch fills the chip; FP32, us for 1 / 2 / 3 / 4 chunks: 2048 sites
+        // 148 / 154 / 166 / 177, 512 sites 51.5 / 45.9 / 47.3 / 47.4, 128 sites 19.2 / 16.6 / 15.2 / 15.4
+        const int chunks = d.S >= 1024 ? 1 : d.S >= 256 ? 2 : 3, chunk = (planes + chunks - 1) / chunks;
+        constexpr int smem = stream::CYT_STAGES * (NI + NCP) * stream::cyt_planes<sizeof(R)>() * 25 * ((25 + V - 1) / V * V) * (int)sizeof(R);
+        auto kern = stream::k_cyto_t<R, NI, NCP, V, 25, stream::CYT_STAGES>;
+        if (!d.st_cyt_ready) {
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return e;
+            d.st_cyt_ready = true;
+        }
+        kern<<<dim3(d.S, chunks), stream::CY_THREADS + 32, smem, st>>>(cy_constants<R>(d), chunk, in, out, d.cin, d.err_flag);
+        return cudaGetLastError();
     }
-    const int bps = (d.m.mc * d.m.mc + stream::CY_THREADS - 1) / stream::CY_THREADS;
-    stream::k_cyto_s<R, NI, NCP><<<bps * d.S, stream::CY_THREADS, 0, st>>>(d.m, d.nc, bps, (const R*)d.cyto[d.ccur],
-                                                                           (R*)d.cyto[1 - d.ccur], d.cin);
+    const int per = (d.m.mc * d.m.cpx / V + stream::CY_THREADS - 1) / stream::CY_THREADS;
+    stream::k_cyto_v<R, NI, NCP, V><<<dim3(d.S, per), stream::CY_THREADS, 0, st>>>(cy_constants<R>(d), in, out, d.cin);
+    return cudaGetLastError();
 }
 
 template <typename R, int NI>
-void launch_cyto_np(cb_dev& d, cudaStream_t st) {
+cudaError_t launch_cyto_np(cb_dev& d, cudaStream_t st) {
     switch (d.m.c_n_pairs) {
-    case 0: launch_cyto_s<R, NI, 0>(d, st); break;
-    case 1: launch_cyto_s<R, NI, 1>(d, st); break;
-    case 2: launch_cyto_s<R, NI, 2>(d, st); break;
-    case 3: launch_cyto_s<R, NI, 3>(d, st); break;
-    default: launch_cyto_s<R, NI, 4>(d, st); break;
+    case 0: return launch_cyto_s<R, NI, 0>(d, st);
+    case 1: return launch_cyto_s<R, NI, 1>(d, st);
+    case 2: return launch_cyto_s<R, NI, 2>(d, st);
+    case 3: return launch_cyto_s<R, NI, 3>(d, st);
+    default: return launch_cyto_s<R, NI, 4>(d, st);
     }
 }
 
@@ -594,8 +750,8 @@ cudaError_t launch_step(cb_dev& d, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     if ((e0 = mark(1)) != cudaSuccess) return e0;
     if (d.m.cyto_type == CB_CYTO_RD3D) {
         if (fast) {
-            if (d.m.n_ions == 1) launch_cyto_np<R, 1>(d, st);
-            else launch_cyto_np<R, 2>(d, st);
+            e0 = d.m.n_ions == 1 ? launch_cyto_np<R, 1>(d, st) : launch_cyto_np<R, 2>(d, st);
+            if (e0 != cudaSuccess) return e0;
         } else {
             dim3 g((d.nc + 255) / 256, d.S);
             k_cyto<R><<<g, 256, 0, st>>>(d.m, d.nc, (const R*)d.cyto[d.ccur], (R*)d.cyto[1 - d.ccur], d.cin);
@@ -604,8 +760,8 @@ cudaError_t launch_step(cb_dev& d, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     }
     if ((e0 = mark(2)) != cudaSuccess) return e0;
     if (fast) {
-        if (d.m.n_ions == 1) launch_rd_np<R, 1>(d, st);
-        else launch_rd_np<R, 2>(d, st);
+        e0 = d.m.n_ions == 1 ? launch_rd_np<R, 1>(d, st) : launch_rd_np<R, 2>(d, st);
+        if (e0 != cudaSuccess) return e0;
     } else {
         dim3 g((d.max_nodes + 255) / 256, d.S);
         k_rd<R><<<g, 256, 0, st>>>(d.m, d.sites, (const R*)d.fields[d.cur], (R*)d.fields[1 - d.cur], (const R*)d.curgrid);
@@ -631,7 +787,7 @@ __global__ void k_sg_features(int S, int n_buf, int max_ch, int ld, const cb_sit
     const float hx = 0.5f * (st.nx - 1), hy = 0.5f * (st.ny - 1);
     for (int c = 0; c < st.n_ch && c < max_ch; ++c) {
         const int node = ch_node[st.ch_off + c];
-        const int gx = node % st.nx, gy = (node / st.nx) % st.ny;
+        const int gx = node % st.px, gy = (node / st.px) % st.ny;
         row[3 * c] = (float)ch_state[st.ch_off + c];
         row[3 * c + 1] = (gx - hx) / hx;
         row[3 * c + 2] = (gy - hy) / hy;

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
     unsigned short* chidx = (unsigned short*)(smem + a.off_chidx);  // 1 + owning RyR at a node, 0 if none
     int* chn = (int*)(smem + a.off_chn);   // local node of own RyRs, -1 otherwise
     int* chs = (int*)(smem + a.off_chs);   // state of every RyR of the site
-    int* cho = (int*)(smem + a.off_cho);   // site node (x + nx*(y + ny*z)) | owner flag in bit 30
+    int* cho = (int*)(smem + a.off_cho);   // stored site node (x + px*(y + ny*z)) | owner flag in bit 30
     int* chr = (int*)(smem + a.off_chr);   // rim index of own RyRs on the rim, -1 otherwise
     R* ftab = (R*)(smem + a.off_ftab);     // [(1 + max_ch)][NI]: RyR currents, slot 0 is zero
     double* pg = (double*)(smem + a.off_pg);      // [2][max_ch] transition probability of each RyR at the next gating
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         if (qsite >= a.S) break;
         const int s = a.order[qsite];
         const cb_site st = a.sites[s];
-        const int nx = st.nx, ny = st.ny, nz = st.nz, nxy = nx * ny, np = st.npad;
+        const int nx = st.nx, ny = st.ny, nz = st.nz, np = st.npad;
         const int nch = st.n_ch;
         const int zmax = NZ == 1 ? 1 : nz - 1;
         const int lo = row_lo(a.rw, rank, ny, C), hi = row_lo(a.rw, rank + 1, ny, C);
@@ -275,11 +275,14 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         // ---------------------------------------------------------- load
         {
             const R* g = (const R*)a.fields + st.node_base * F;
+            const int px = st.px;
+            const fastdiv fd_nx = make_fastdiv(nx);
             for (int f = 0; f < FP; ++f)
                 for (int z = 0; z < nz; ++z) {
-                    const R* src = g + (long long)f * np + (long long)nx * (slo + (long long)ny * z);
+                    const R* src = g + (long long)f * np + (long long)px * (slo + (long long)ny * z);
                     for (int k = tid; k < lstride; k += blockDim.x) {
-                        const R v = f < F ? src[k] : (R)0;  // unused species slots hold zeros
+                        // stored rows have pitch px, rows in shared memory nx
+                        const R v = f < F ? src[k + fdiv(k, fd_nx) * (px - nx)] : (R)0;  // unused species slots hold zeros
                         fa[f * cap + lstride * z + k] = v;
                         fb[f * cap + lstride * z + k] = v;
                     }
@@ -293,13 +296,17 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                 const R* cs = (const R*)a.cyto + (size_t)s * CS * nc;
                 for (int c = 0; c < CSM; ++c)
                     for (int k = tid; k < cloc; k += blockDim.x) {
-                        const R v = c < CS ? cs[(size_t)c * nc + (size_t)splo * mc2 + k] : (R)0;
+                        const int row = k / mc;  // stored rows have pitch cpx, rows in shared memory mc
+                        const R v = c < CS ? cs[(size_t)c * nc + (size_t)(splo * mc + row) * m.cpx + (k - row * mc)] : (R)0;
                         const int pl = k / mc2, l = pl * cps + (k - pl * mc2);
                         ca[c * ccap + l] = v;
                         cb[c * ccap + l] = v;
                     }
                 const int nrim = cb_rim_count(nx, ny);
-                for (int k = tid; k < nrim; k += blockDim.x) crim[k] = (unsigned short)a.rim_cnode[st.rim_off + k];
+                for (int k = tid; k < nrim; k += blockDim.x) {
+                    const int cn = a.rim_cnode[st.rim_off + k], jj = cn / m.cpx;
+                    crim[k] = (unsigned short)(cn - jj * (m.cpx - mc));
+                }
                 for (int k = tid; k < mc2; k += blockDim.x) slot_of[k] = 0xFFFF;
                 const int* gp = a.dep_ptr + (size_t)s * (mc2 + 1);
                 for (int k = tid; k <= mc2; k += blockDim.x) dptr[k] = (unsigned short)gp[k];
@@ -380,7 +387,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         }
         for (int c = tid; c < nch; c += blockDim.x) {
             const int gnode = a.ch_node[st.ch_off + c];
-            const int x = gnode % nx, y = (gnode / nx) % ny, z = gnode / nxy;
+            const int px = st.px, x = gnode % px, y = (gnode / px) % ny, z = gnode / (px * ny);
             chs[c] = a.ch_state[st.ch_off + c];
             const bool owner = a.ch_owner[st.ch_off + c] != 0;
             cho[c] = gnode | (owner ? (1 << 30) : 0);
@@ -1073,11 +1080,13 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         __syncthreads();
         {
             R* g = (R*)a.fields + st.node_base * F;
+            const int px = a.sites[s].px;  // read again: not kept over the step loop
+            const fastdiv fd_nx = make_fastdiv(nx);
             for (int f = 0; f < F; ++f)
                 for (int z = 0; z < nz; ++z) {
-                    R* dst = g + (long long)f * np + (long long)nx * (lo + (long long)ny * z);
+                    R* dst = g + (long long)f * np + (long long)px * (lo + (long long)ny * z);
                     const R* src = fa + f * cap + lstride * z + nx * (lo - slo);
-                    for (int k = tid; k < nx * (hi - lo); k += blockDim.x) dst[k] = src[k];
+                    for (int k = tid; k < nx * (hi - lo); k += blockDim.x) dst[k + fdiv(k, fd_nx) * (px - nx)] = src[k];
                 }
             if (rank == 0) {
                 const unsigned int* qs = (const unsigned int*)&q;
@@ -1093,8 +1102,8 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                 R* cd = (R*)a.cyto + (size_t)s * CS * nc;
                 for (int c = 0; c < CS; ++c)
                     for (int k = tid; k < (phi - plo) * mc2; k += blockDim.x) {
-                        const int pl = k / mc2;
-                        cd[(size_t)c * nc + (size_t)plo * mc2 + k] = ca[c * ccap + (plo - splo + pl) * cps + (k - pl * mc2)];
+                        const int pl = k / mc2, row = k / mc;
+                        cd[(size_t)c * nc + (size_t)(plo * mc + row) * m.cpx + (k - row * mc)] = ca[c * ccap + (plo - splo + pl) * cps + (k - pl * mc2)];
                     }
                 if (rank == r0 && a.nsteps > 0) {
                     // deposit of the final Update, for the next launch
