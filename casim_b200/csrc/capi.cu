@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -97,6 +98,28 @@ casim_status set_err(casim_b200_sim* h, casim_status s, const std::string& msg) 
         return set_err(h, CASIM_EINVAL, e.what());                          \
     }
 
+// Error words that kernels with bounded waits set, in mapped host memory so that a check costs no
+// copy. Page-locking takes milliseconds, so handles share pages of words: each takes a free one and
+// gives it back; a page is allocated when all words of the earlier ones are taken.
+std::mutex g_flag_lock;
+std::vector<int*> g_flags;
+int* take_flag() {
+    std::lock_guard<std::mutex> g(g_flag_lock);
+    if (g_flags.empty()) {
+        int* p = nullptr;
+        ck(cudaHostAlloc((void**)&p, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+        for (int i = 0; i < 1024; ++i) g_flags.push_back(p + i);
+    }
+    int* f = g_flags.back();
+    g_flags.pop_back();
+    *f = 0;
+    return f;
+}
+void give_flag(int* f) {
+    std::lock_guard<std::mutex> g(g_flag_lock);
+    g_flags.push_back(f);
+}
+
 // a kernel's bounded wait for its own copies ran out in an earlier launch (the state is not valid)
 bool wait_gave_up(casim_b200_sim* h) {
     if (!h->d.err_host || !*(volatile int*)h->d.err_host) return false;
@@ -127,7 +150,8 @@ void build_device(casim_b200_sim* h, int precision) {
     std::vector<cb_site> sites(d.S);
     std::vector<int> ch_node, ch_owner;
     std::vector<cb_site_scalars> sc(d.S);
-    std::vector<int> rim_cnode, dep_ptr, dep_term;
+    std::vector<int> rim_cnode, dep_ptr, dep_term, dep_pos, dep_nptr(1, 0);
+    std::vector<int3> dep_node;
     long long nb = 0;
     int choff = 0, rimoff = 0, termoff = 0;
     const int mc = cfg.m.mc;
@@ -191,6 +215,15 @@ void build_device(casim_b200_sim* h, int precision) {
                 acc += (int)lists[cn].size();
             }
             dep_ptr.push_back(acc);
+            // the same lists for the specialised Update: the place of each term in the grouped order,
+            // and the receiving nodes
+            dep_pos.resize((size_t)termoff + acc);
+            const int* p = dep_ptr.data() + dep_ptr.size() - (size_t)(mc * mc + 1);
+            for (int k = 0; k < acc; ++k) dep_pos[(size_t)termoff + dep_term[(size_t)termoff + k]] = k;
+            for (int cn = 0; cn < mc * mc; ++cn)
+                if (p[cn + 1] > p[cn]) dep_node.push_back(make_int3(cn, p[cn], p[cn + 1]));
+            d.st_max_dn = std::max(d.st_max_dn, (int)dep_node.size() - dep_nptr.back());
+            dep_nptr.push_back((int)dep_node.size());
             termoff += acc;
         }
     }
@@ -225,15 +258,16 @@ void build_device(casim_b200_sim* h, int precision) {
         d.rim_cnode = dupload(h, rim_cnode);
         d.dep_ptr = dupload(h, dep_ptr);
         d.dep_term = dupload(h, dep_term);
+        d.st_dpos = dupload(h, dep_pos);
+        d.st_dnptr = dupload(h, dep_nptr);
+        d.st_dnode = dupload(h, dep_node);
     }
     for (int w = 0; w < 2; ++w)
         if (!cfg.sp_x[w].empty()) {
             d.spx[w] = dupload(h, cfg.sp_x[w]);
             d.spc[w] = dupload(h, cfg.sp_c[w]);
         }
-    // kernels with bounded waits set it; in host memory so that a check costs no copy
-    ck(cudaHostAlloc((void**)&d.err_host, sizeof(int), cudaHostAllocMapped), "cudaHostAlloc");
-    *d.err_host = 0;
+    d.err_host = take_flag();
     ck(cudaHostGetDevicePointer((void**)&d.err_flag, d.err_host, 0), "cudaHostGetDevicePointer");
 }
 
@@ -317,8 +351,9 @@ casim_status casim_b200_destroy(casim_h h) {
     if (h->d.rs_counter) cudaFree(h->d.rs_counter);
     if (h->d.rs_pow2) cudaFree(h->d.rs_pow2);
     if (h->d.st_tiles) cudaFree(h->d.st_tiles);
-    if (h->d.st_runs) cudaFree(h->d.st_runs);
-    if (h->d.err_host) cudaFreeHost(h->d.err_host);
+    for (void* p : {h->d.st_runs, (void*)h->d.st_prob, (void*)h->d.st_ch})
+        if (p) cudaFree(p);
+    if (h->d.err_host) give_flag(h->d.err_host);
     if (h->d.st_chcol) cudaFree(h->d.st_chcol);
     if (h->d.pre_jump) cudaFree(h->d.pre_jump);
     cb_resident_free(h->d);

@@ -67,7 +67,13 @@ struct cb_dev {
     cb_gate* gates = nullptr;
     int* site_gate = nullptr;
     int n_gates = 0;
-    unsigned long long* pre_jump = nullptr;  // k_pre_r: MRG32k3a jumps A^(2l), l < 32
+    unsigned long long* pre_jump = nullptr;  // warp-parallel gating: MRG32k3a jumps A^(2l), l < 32
+    int2* st_ch = nullptr;       // per RyR: node, flags (stream::CH_*)
+    double* st_prob = nullptr;   // transition probability per RyR (60-state: then mouth Ca and Mg), within one step call
+    int* st_dpos = nullptr;      // RD3D deposits of the specialised Update (stream::dep_args)
+    int* st_dnptr = nullptr;
+    int3* st_dnode = nullptr;
+    int st_max_dn = 0;           // largest receiving-node count of a site
 };
 
 // plain path (plain.cu)

@@ -409,6 +409,35 @@ __global__ void __launch_bounds__(256) k_update(cb_model m, int NS, const cb_sit
         }
 }
 
+// jump table of the warp-parallel gating: row l < 32 holds A^(2l), both components, stored
+// entry-major (row 31, A^62, also takes a lane from one chunk of 32 draws to the next)
+bool pre_jump(cb_dev& d) {
+    if (d.pre_jump) return true;
+    std::vector<unsigned long long> t(32 * 18);
+    const cbrng::Mat3 a1 = cbrng::step_matrix1(), a2 = cbrng::step_matrix2();
+    cbrng::Mat3 p1{{{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}}, p2 = p1;  // A^(2l)
+    for (int l = 0; l < 32; ++l) {
+        for (int i = 0; i < 9; ++i) {
+            t[32 * i + l] = p1.a[i / 3][i % 3];
+            t[32 * (9 + i) + l] = p2.a[i / 3][i % 3];
+        }
+        for (int k = 0; k < 2; ++k) {
+            p1 = cbrng::matmul(a1, p1, cbrng::M1);
+            p2 = cbrng::matmul(a2, p2, cbrng::M2);
+        }
+    }
+    if (cudaMalloc(&d.pre_jump, sizeof(unsigned long long) * t.size()) != cudaSuccess) {
+        d.pre_jump = nullptr;
+        return false;
+    }
+    if (cudaMemcpy(d.pre_jump, t.data(), sizeof(unsigned long long) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaFree(d.pre_jump);
+        d.pre_jump = nullptr;
+        return false;
+    }
+    return true;
+}
+
 // The specialised stencils (stream_kernels.cuh) serve 1-2 ions with up to 4 pairs
 // and a cleft of one layer (2D) or three (3D) at every site; the first step lists
 // the cleft blocks (site, first group). Returns the tile count, 0 if not covered.
@@ -473,6 +502,20 @@ int stream_tiles(cb_dev& d) {
         }
     if (cudaMalloc(&d.st_chcol, sizeof(unsigned) * bits.size()) != cudaSuccess) return 0;
     if (cudaMemcpy(d.st_chcol, bits.data(), sizeof(unsigned) * bits.size(), cudaMemcpyHostToDevice) != cudaSuccess) return 0;
+    if (!pre_jump(d)) return 0;
+    // per RyR its node and flags
+    std::vector<int2> chv((size_t)d.total_ch);
+    std::vector<int> own((size_t)d.total_ch);
+    if (d.total_ch && cudaMemcpy(own.data(), d.ch_owner, sizeof(int) * own.size(), cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
+    for (int s = 0; s < d.S; ++s)
+        for (int c = hs[s].ch_off; c < hs[s].ch_off + hs[s].n_ch; ++c) {
+            const int x = chn[c] % hs[s].px, y = (chn[c] / hs[s].px) % hs[s].ny;
+            const bool rim = x == 0 || x == hs[s].nx - 1 || y == 0 || y == hs[s].ny - 1;
+            chv[c] = make_int2(chn[c], (own[c] ? stream::CH_OWNER : 0) | (rim ? stream::CH_RIM : 0));
+        }
+    if (cudaMalloc(&d.st_ch, sizeof(int2) * std::max<size_t>(chv.size(), 1)) != cudaSuccess) return 0;
+    if (cudaMemcpy(d.st_ch, chv.data(), sizeof(int2) * chv.size(), cudaMemcpyHostToDevice) != cudaSuccess) return 0;
+    if (cudaMalloc(&d.st_prob, sizeof(double) * (size_t)std::max<long long>(d.total_ch, 1) * (d.mwc ? 3 : 1)) != cudaSuccess) return 0;
     // shared-memory carve of the asynchronous kernel's stages. It is used where at least two
     // blocks (FP64) or three (FP32) fit an SM, 12 computing warps; with fewer it is no faster than
     // k_rd_v (2048 sites, FP32: three blocks 189 us, two 270, k_rd_v 262)
@@ -506,69 +549,71 @@ int stream_tiles(cb_dev& d) {
     return d.st_ntiles;
 }
 
-// jump table of k_pre_r: row l < 32 holds A^(2l), both components (row 31, A^62, also
-// takes a lane from one chunk of 32 draws to the next)
-bool pre_jump(cb_dev& d) {
-    if (d.pre_jump) return true;
-    std::vector<unsigned long long> t(32 * 18);
-    const cbrng::Mat3 a1 = cbrng::step_matrix1(), a2 = cbrng::step_matrix2();
-    cbrng::Mat3 p1{{{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}}, p2 = p1;  // A^(2l)
-    for (int l = 0; l < 32; ++l) {
-        for (int i = 0; i < 9; ++i) {
-            t[18 * l + i] = p1.a[i / 3][i % 3];
-            t[18 * l + 9 + i] = p2.a[i / 3][i % 3];
-        }
-        for (int k = 0; k < 2; ++k) {
-            p1 = cbrng::matmul(a1, p1, cbrng::M1);
-            p2 = cbrng::matmul(a2, p2, cbrng::M2);
-        }
-    }
-    if (cudaMalloc(&d.pre_jump, sizeof(unsigned long long) * t.size()) != cudaSuccess) {
-        d.pre_jump = nullptr;
-        return false;
-    }
-    if (cudaMemcpy(d.pre_jump, t.data(), sizeof(unsigned long long) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(d.pre_jump);
-        d.pre_jump = nullptr;
-        return false;
-    }
-    return true;
+stream::gate_args gating(const cb_dev& d) {
+    stream::gate_args g{};
+    g.spx0 = d.spx[0];
+    g.spc0 = d.spc[0];
+    g.spx1 = d.spx[1];
+    g.spc1 = d.spc[1];
+    g.J = d.pre_jump;
+    g.gates = d.gates;
+    g.site_gate = d.site_gate;
+    g.mwc = d.mwc;
+    g.ch_state = d.ch_state;
+    g.ch_micro = d.ch_micro;
+    g.prob = d.st_prob;
+    g.pcm = d.st_prob + d.total_ch;
+    return g;
 }
 
+// gate: a time step's gating, pools and Update, right after the cleft kernel; else the Update alone
 template <typename R, int NI, int NP, bool RD3D>
-cudaError_t launch_update_s(cb_dev& d, cudaStream_t st, bool after_step) {
-    size_t smem = 8 * (NI + NP + NI) * sizeof(double);
-    if (RD3D) smem += (size_t)d.max_terms * (NI + NP) * sizeof(double) + sizeof(int) * ((size_t)d.m.mc * d.m.mc + 1 + d.max_terms);
-    auto kern = stream::k_update_s<R, NI, NP, RD3D>;
-    if (smem > 48 * 1024) {
+cudaError_t launch_update_s(cb_dev& d, cudaStream_t st, bool gate, bool want) {
+    stream::dep_args dep{};
+    if (RD3D) {
+        dep.pos = d.st_dpos;
+        dep.node_ptr = d.st_dnptr;
+        dep.node = d.st_dnode;
+        dep.max_nodes = d.st_max_dn;
+        for (int c = 0; c < d.CS; ++c) {
+            const int p = c < NI ? -1 : d.m.c_dyad_pair[c - NI];
+            if (c >= NI && p < 0) continue;
+            dep.f[dep.n] = c < NI ? c : NI + p;
+            dep.c[dep.n++] = c;
+        }
+    }
+    size_t smem = (size_t)(d.max_ch + 7) / 8 * 8;
+    if (RD3D) smem += (size_t)d.max_terms * dep.n * sizeof(double) + (size_t)dep.max_nodes * sizeof(int3);
+    auto kern = gate ? stream::k_update_s<R, NI, NP, RD3D, true> : stream::k_update_s<R, NI, NP, RD3D, false>;
+    if (smem > 40 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    kern<<<d.S, stream::UP_THREADS, smem, st>>>(d.m, d.NS, d.sites, (R*)d.fields[d.cur], (R*)d.curgrid, d.ch_node, d.ch_owner, d.ch_state,
-                                                d.mouth, d.sc, d.nc, (const R*)d.cyto[1 - d.ccur], d.cin, d.rim_cnode, d.dep_ptr,
-                                                d.dep_term, after_step ? (const R*)d.fields[1 - d.cur] : nullptr, d.max_terms);
+    // the rim reads the cytosol as it was before its latest step (RD3D coupling)
+    kern<<<d.S, stream::UP_THREADS, smem, st>>>(d.m, gating(d), dep, d.NS, want, d.sites, (R*)d.fields[d.cur], (const R*)d.fields[1 - d.cur],
+                                                (R*)d.curgrid, d.st_ch, d.mouth, d.sc, d.nc, (const R*)d.cyto[1 - d.ccur], d.cin, d.rim_cnode,
+                                                d.max_ch, d.max_terms);
     return cudaGetLastError();
 }
 
 template <typename R, int NI, bool RD3D>
-cudaError_t launch_update_np(cb_dev& d, cudaStream_t st, bool after_step) {
+cudaError_t launch_update_np(cb_dev& d, cudaStream_t st, bool gate, bool want) {
     switch (d.m.n_pairs) {
-    case 0: return launch_update_s<R, NI, 0, RD3D>(d, st, after_step);
-    case 1: return launch_update_s<R, NI, 1, RD3D>(d, st, after_step);
-    case 2: return launch_update_s<R, NI, 2, RD3D>(d, st, after_step);
-    case 3: return launch_update_s<R, NI, 3, RD3D>(d, st, after_step);
-    default: return launch_update_s<R, NI, 4, RD3D>(d, st, after_step);
+    case 0: return launch_update_s<R, NI, 0, RD3D>(d, st, gate, want);
+    case 1: return launch_update_s<R, NI, 1, RD3D>(d, st, gate, want);
+    case 2: return launch_update_s<R, NI, 2, RD3D>(d, st, gate, want);
+    case 3: return launch_update_s<R, NI, 3, RD3D>(d, st, gate, want);
+    default: return launch_update_s<R, NI, 4, RD3D>(d, st, gate, want);
     }
 }
 
-// after_step: right after k_rd_v, which set the rim already
 template <typename R>
-cudaError_t launch_update(cb_dev& d, cudaStream_t st, bool after_step = false) {
+cudaError_t launch_update(cb_dev& d, cudaStream_t st, bool gate = false, bool want = true) {
     if (stream_tiles(d) > 0) {
         const bool rd3d = d.m.cyto_type == CB_CYTO_RD3D;
         if (d.m.n_ions == 1)
-            return rd3d ? launch_update_np<R, 1, true>(d, st, after_step) : launch_update_np<R, 1, false>(d, st, after_step);
-        return rd3d ? launch_update_np<R, 2, true>(d, st, after_step) : launch_update_np<R, 2, false>(d, st, after_step);
+            return rd3d ? launch_update_np<R, 1, true>(d, st, gate, want) : launch_update_np<R, 1, false>(d, st, gate, want);
+        return rd3d ? launch_update_np<R, 2, true>(d, st, gate, want) : launch_update_np<R, 2, false>(d, st, gate, want);
     }
     size_t smem = 256 * sizeof(double);
     if (d.m.cyto_type == CB_CYTO_RD3D) smem += (size_t)d.max_terms * d.m.F * sizeof(double);
@@ -656,7 +701,7 @@ cudaError_t launch_rd_s(cb_dev& d, cudaStream_t st) {
     const R* in = (const R*)d.fields[d.cur];
     R* out = (R*)d.fields[1 - d.cur];
     // the cytosol as it was before its latest step (k_cyto flipped ccur already)
-    const R* cy = (const R*)d.cyto[1 - d.ccur];
+    const R* cy = d.m.cyto_type == CB_CYTO_RD3D ? (const R*)d.cyto[1 - d.ccur] : nullptr;
     if (d.st_runs) {
         stream::rd_stage g;
         std::memcpy(&g, d.st_stage, sizeof(g));
@@ -672,11 +717,11 @@ cudaError_t launch_rd_s(cb_dev& d, cudaStream_t st) {
             d.st_grid = std::max(1, std::min(sms * per, d.st_nruns));
         }
         kern<<<d.st_grid, stream::rdt_threads(sizeof(R)) + 32, smem, st>>>(rd_constants<R>(d), g, (const stream::rd_tile*)d.st_runs, d.st_nruns, in,
-                                                                          out, (const R*)d.curgrid, d.sc, cy, d.rim_cnode, d.st_chcol, d.err_flag);
+                                                                          out, (const R*)d.curgrid, cy, d.rim_cnode, d.st_chcol, d.err_flag);
         return cudaGetLastError();
     }
     auto kern = d.st_nz == 1 ? stream::k_rd_v<R, NI, NP, 1, V> : stream::k_rd_v<R, NI, NP, 3, V>;
-    kern<<<d.st_ntiles, stream::RD_THREADS, 0, st>>>(rd_constants<R>(d), d.sites, d.st_tiles, in, out, (const R*)d.curgrid, d.sc, cy,
+    kern<<<d.st_ntiles, stream::RD_THREADS, 0, st>>>(rd_constants<R>(d), d.sites, d.st_tiles, in, out, (const R*)d.curgrid, cy,
                                                      d.rim_cnode, d.st_chcol);
     return cudaGetLastError();
 }
@@ -729,24 +774,23 @@ cudaError_t launch_cyto_np(cb_dev& d, cudaStream_t st) {
     }
 }
 
+// One time step, the `first` or `last` of its call. ev (optional, 5 events): recorded before the
+// gating kernel (specialised kernels: the probabilities of a call's first gating; the gating runs
+// in the Update kernel) and after each of the gating, cytosol, cleft and Update kernels.
 template <typename R>
-// ev (optional, 5 events): recorded before the gating kernel and after each of the
-// gating, cytosol, cleft and Update kernels
-cudaError_t launch_step(cb_dev& d, cudaStream_t st, cudaEvent_t* ev = nullptr) {
+cudaError_t launch_step(cb_dev& d, cudaStream_t st, bool first, bool last, cudaEvent_t* ev = nullptr) {
     auto mark = [&](int k) { return ev ? cudaEventRecord(ev[k], st) : cudaSuccess; };
     cudaError_t e0 = mark(0);
     if (e0 != cudaSuccess) return e0;
     const bool fast = stream_tiles(d) > 0;
-    if (fast && pre_jump(d)) {
-        auto kern = d.mwc ? stream::k_pre_r<true> : stream::k_pre_r<false>;
-        kern<<<(d.S + stream::PRE_WARPS - 1) / stream::PRE_WARPS, 32 * stream::PRE_WARPS, 0, st>>>(
-            d.m, d.S, d.NS, d.sites, d.sc, d.ch_state, d.mouth, d.spx[0], d.spc[0], d.spx[1], d.spc[1], d.pre_jump, d.gates,
-            d.site_gate, d.ch_micro, d.mwc);
-    } else if (d.site_gate)
-        return cudaErrorNotSupported;  // per-site models need k_pre_r
-    else
+    if (fast) {
+        if (first) stream::k_prob<<<d.S, 64, 0, st>>>(d.m, gating(d), d.NS, d.sites, d.mouth);
+    } else if (d.site_gate) {
+        return cudaErrorNotSupported;  // per-site models need the specialised kernels
+    } else {
         k_pre<<<(d.S + 127) / 128, 128, 0, st>>>(d.m, d.S, d.NS, d.sites, d.sc, d.ch_state, d.mouth, d.spx[0], d.spc[0],
                                                    d.spx[1], d.spc[1], d.ch_micro, d.mwc);
+    }
     if ((e0 = mark(1)) != cudaSuccess) return e0;
     if (d.m.cyto_type == CB_CYTO_RD3D) {
         if (fast) {
@@ -768,7 +812,7 @@ cudaError_t launch_step(cb_dev& d, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     }
     d.cur ^= 1;
     if ((e0 = mark(3)) != cudaSuccess) return e0;
-    if ((e0 = launch_update<R>(d, st, fast)) != cudaSuccess) return e0;
+    if ((e0 = launch_update<R>(d, st, fast, last)) != cudaSuccess) return e0;
     return mark(4);
 }
 
@@ -904,18 +948,20 @@ cudaError_t cb_plain_update(cb_dev& d, cudaStream_t st, long long* launches) {
 
 bool cb_plain_streaming(cb_dev& d) { return stream_tiles(d) > 0; }
 
-bool cb_plain_gating_ready(cb_dev& d) { return stream_tiles(d) > 0 && !d.mwc && pre_jump(d); }
+bool cb_plain_gating_ready(cb_dev& d) { return stream_tiles(d) > 0 && !d.mwc; }
 
 cudaError_t cb_plain_step_marked(cb_dev& d, cudaStream_t st, cudaEvent_t* ev) {
-    return d.precision == 0 ? launch_step<double>(d, st, ev) : launch_step<float>(d, st, ev);
+    return d.precision == 0 ? launch_step<double>(d, st, true, true, ev) : launch_step<float>(d, st, true, true, ev);
 }
 
 cudaError_t cb_plain_step(cb_dev& d, long long n, cudaStream_t st, long long* launches) {
-    const int per = 3 + (d.m.cyto_type == CB_CYTO_RD3D ? 1 : 0);
+    const bool fast = stream_tiles(d) > 0;
+    const int per = (fast ? 2 : 3) + (d.m.cyto_type == CB_CYTO_RD3D ? 1 : 0);
     for (long long i = 0; i < n; ++i) {
-        cudaError_t e = d.precision == 0 ? launch_step<double>(d, st) : launch_step<float>(d, st);
+        const bool first = i == 0, last = i == n - 1;
+        cudaError_t e = d.precision == 0 ? launch_step<double>(d, st, first, last) : launch_step<float>(d, st, first, last);
         if (e != cudaSuccess) return e;
-        if (launches) *launches += per;
+        if (launches) *launches += per + (fast && first ? 1 : 0);
     }
     return cudaSuccess;
 }

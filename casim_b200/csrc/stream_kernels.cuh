@@ -48,10 +48,12 @@ __device__ __forceinline__ group<R, V> load_group(const R* p) {
 }
 // outputs are read back only in the next time step, after the whole state has passed
 // through L2: cache-streaming stores leave L2 to the rows neighbouring blocks read
+// (keep: nodes that the Update reads right after the step)
 template <int V, typename R>
-__device__ __forceinline__ void store_group(R* p, const group<R, V>& g) {
+__device__ __forceinline__ void store_group(R* p, const group<R, V>& g, bool keep = false) {
     typedef typename word_of<R, V>::T W;
-    __stcs((W*)p, *(const W*)&g);
+    if (keep) *(W*)p = *(const W*)&g;
+    else __stcs((W*)p, *(const W*)&g);
 }
 
 // a model constant, twice: a packed operand of two nodes
@@ -225,15 +227,13 @@ __device__ __forceinline__ void node_reactions(const rd_const<R>& k, const group
 }
 
 // Cleft step of the groups [tile.y, tile.y + 256) of site tile.x (tile.z, tile.w: the
-// division by the row pitch). The rim takes the Dirichlet values that the Update would set
-// right after this step (CaSim/DyadRD2DCPU.cpp:274-303), from the same sources: the cytosol as
-// it was before its latest step (cyto, RD3D) or the pool values of this step (sc); the Update
-// then leaves the rim alone (k_update_s with prev set).
+// division by the row pitch). With the RD3D cytosol the rim takes the Dirichlet values of this
+// step's Update (CaSim/DyadRD2DCPU.cpp:274-303), the cytosol as it was before its latest step; with
+// the pool (cyto null) it carries its values over and the Update sets it.
 template <typename R, int NI, int NP, int NZ, int V>
 __global__ void __launch_bounds__(RD_THREADS, rd_min_blocks(sizeof(R), NI + NP, NZ, V))
     k_rd_v(const __grid_constant__ rd_const<R> k, const cb_site* __restrict__ sites, const int4* __restrict__ tiles,
-           const R* __restrict__ in, R* __restrict__ out, const R* __restrict__ curg, const cb_site_scalars* __restrict__ sc,
-           const R* __restrict__ cyto, const int* __restrict__ rim_cnode, const unsigned* __restrict__ chcol) {
+           const R* __restrict__ in, R* __restrict__ out, const R* __restrict__ curg, const R* __restrict__ cyto, const int* __restrict__ rim_cnode, const unsigned* __restrict__ chcol) {
     constexpr int F = NI + NP;
     const int4 tl = tiles[blockIdx.x];
     const cb_site st = sites[tl.x];
@@ -244,17 +244,19 @@ __global__ void __launch_bounds__(RD_THREADS, rd_min_blocks(sizeof(R), NI + NP, 
     R* __restrict__ o = out + st.node_base * F + col;
     const int y = (int)((__umulhi((unsigned)col, (unsigned)tl.z) + (unsigned)col) >> tl.w), x = col - y * px;
     auto rim_values = [&](int ri, R(&b)[F]) {
-        if (cyto) {
-            const R* cy = cyto + (long long)tl.x * k.CS * k.nc + rim_cnode[st.rim_off + ri];
+        const R* cy = cyto + (long long)tl.x * k.CS * k.nc + rim_cnode[st.rim_off + ri];
 #pragma unroll
-            for (int f = 0; f < F; ++f) b[f] = k.src[f] >= 0 ? cy[k.src[f] * k.nc] : k.init[f];
-        } else {
-            const cb_site_scalars& q = sc[tl.x];
-#pragma unroll
-            for (int f = 0; f < F; ++f) b[f] = (R)(f < NI ? q.c_ions[f < NI ? f : 0] : q.c_bnd[f < NI ? 0 : f - NI]);
-        }
+        for (int f = 0; f < F; ++f) b[f] = k.src[f] >= 0 ? cy[k.src[f] * k.nc] : k.init[f];
     };
+    const bool carry = cyto == nullptr;
     if (y == 0 || y == ny - 1) {
+        if (carry) {
+#pragma unroll
+            for (int f = 0; f < F; ++f)
+#pragma unroll
+                for (int z = 0; z < NZ; ++z) store_group(o + f * np + z * pxy, load_group<V>(u + f * np + z * pxy));
+            return;
+        }
 #pragma unroll
         for (int e = 0; e < V; ++e) {
             R b[F];
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(RD_THREADS, rd_min_blocks(sizeof(R), NI + NP, 
     // values are loaded first and put in last
     const bool edge = x == 0 || x + V >= nx;
     R b[F];
-    if (edge) rim_values(x == 0 ? y : ny + y, b);
+    if (edge && !carry) rim_values(x == 0 ? y : ny + y, b);
     // RyR currents exist only in the columns that hold a RyR (bits of the site's words in
     // chcol), in layer 0; elsewhere the current grid is zero and is not read
     const long long bit = st.node_base + col;
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(RD_THREADS, rd_min_blocks(sizeof(R), NI + NP, 
             group<R, V> w = gadd(c[f][z], evo[f]);
 #pragma unroll
             for (int e = 0; e < V; ++e)
-                if (edge && (x + e == 0 || x + e >= nx - 1)) w.v[e] = b[f];
+                if (edge && (x + e == 0 || x + e >= nx - 1)) w.v[e] = carry ? c[f][z].v[e] : b[f];
             store_group(o + f * np + z * pxy, w);
         }
     }
@@ -377,8 +379,7 @@ struct rd_stage {
 template <typename R, int NI, int NP, int NZ, int V, int STAGES>
 __global__ void __launch_bounds__(rdt_threads(sizeof(R)) + 32, rdt_blocks(sizeof(R), NI + NP, NZ))
     k_rd_t(const __grid_constant__ rd_const<R> k, const __grid_constant__ rd_stage g, const rd_tile* __restrict__ tiles, int ntiles,
-           const R* __restrict__ in, R* __restrict__ out, const R* __restrict__ curg, const cb_site_scalars* __restrict__ sc,
-           const R* __restrict__ cyto, const int* __restrict__ rim_cnode, const unsigned* __restrict__ chcol, int* __restrict__ err) {
+           const R* __restrict__ in, R* __restrict__ out, const R* __restrict__ curg, const R* __restrict__ cyto, const int* __restrict__ rim_cnode, const unsigned* __restrict__ chcol, int* __restrict__ err) {
     constexpr int F = NI + NP, THREADS = rdt_threads(sizeof(R)), TN = THREADS * V, EXT = 16 / (int)sizeof(R);
     extern __shared__ __align__(128) unsigned char rd_smem[];
     __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES];
@@ -433,20 +434,14 @@ __global__ void __launch_bounds__(rdt_threads(sizeof(R)) + 32, rdt_blocks(sizeof
             const int ce = tl.col0 + n - 1;
             const int y1 = (int)((__umulhi((unsigned)ce, tl.mul) + (unsigned)ce) >> tl.sh);
             const int side = 2 * (y1 - y0 + 1), top = y0 == 0 ? tl.nx : 0, bot = y1 == tl.ny - 1 ? tl.nx : 0;
-            for (int i = lane; i < side + top + bot; i += 32) {
+            for (int i = cyto ? lane : INT_MAX; i < side + top + bot; i += 32) {
                 int ri;
                 if (i < side) ri = (i & 1 ? tl.ny : 0) + y0 + (i >> 1);
                 else if (i < side + top) ri = cb_rim_index(i - side, 0, tl.nx, tl.ny);
                 else ri = cb_rim_index(i - side - top, tl.ny - 1, tl.nx, tl.ny);
-                if (cyto) {
-                    const R* cy = cyto + (long long)tl.site * k.CS * k.nc + rim_cnode[tl.rim_off + ri];
+                const R* cy = cyto + (long long)tl.site * k.CS * k.nc + rim_cnode[tl.rim_off + ri];
 #pragma unroll
-                    for (int f = 0; f < F; ++f) rv[i * F + f] = k.src[f] >= 0 ? cy[k.src[f] * k.nc] : k.init[f];
-                } else {
-                    const cb_site_scalars& q = sc[tl.site];
-#pragma unroll
-                    for (int f = 0; f < F; ++f) rv[i * F + f] = (R)(f < NI ? q.c_ions[f < NI ? f : 0] : q.c_bnd[f < NI ? 0 : f - NI]);
-                }
+                for (int f = 0; f < F; ++f) rv[i * F + f] = k.src[f] >= 0 ? cy[k.src[f] * k.nc] : k.init[f];
             }
             __syncwarp();
             if (lane == 0) bar_arrive(&full[s]);
@@ -475,7 +470,15 @@ __global__ void __launch_bounds__(rdt_threads(sizeof(R)) + 32, rdt_blocks(sizeof
             const int y = (int)((__umulhi((unsigned)col, tl.mul) + (unsigned)col) >> tl.sh), x = col - y * px;
             const int y0 = (int)((__umulhi((unsigned)col0, tl.mul) + (unsigned)col0) >> tl.sh);
             const R* rv = (const R*)(stg + g.rim);
-            if (y == 0 || y == ny - 1) {
+            const bool carry = cyto == nullptr;
+            if (carry && (y == 0 || y == ny - 1)) {
+#pragma unroll
+                for (int f = 0; f < F; ++f)
+#pragma unroll
+                    for (int z = 0; z < NZ; ++z)
+                        store_group(o + f * np + z * pxy,
+                                    load_group<V>((const R*)(stg + g.plane[f] + z * g.stride[f]) + gi + (k.diff[f] ? g.halo : 0)));
+            } else if (y == 0 || y == ny - 1) {
                 const int ce = min(col0 + TN, pxy) - 1;
                 const int y1 = (int)((__umulhi((unsigned)ce, tl.mul) + (unsigned)ce) >> tl.sh);
                 const R* row = rv + (2 * (y1 - y0 + 1) + (y == 0 || y0 > 0 ? 0 : nx)) * F;
@@ -485,7 +488,7 @@ __global__ void __launch_bounds__(rdt_threads(sizeof(R)) + 32, rdt_blocks(sizeof
 #pragma unroll
                     for (int e = 0; e < V; ++e) w.v[e] = row[min(x + e, nx - 1) * F + f];
 #pragma unroll
-                    for (int z = 0; z < NZ; ++z) store_group(o + f * np + z * pxy, w);
+                    for (int z = 0; z < NZ; ++z) store_group(o + f * np + z * pxy, w, true);
                 }
             } else {
                 const bool has_ch = (((const unsigned*)(stg + g.bits))[gi >> 5] >> (gi & 31)) & ((1u << V) - 1u);
@@ -498,6 +501,7 @@ __global__ void __launch_bounds__(rdt_threads(sizeof(R)) + 32, rdt_blocks(sizeof
                     for (int e = 0; e < V; ++e) cur[j].v[e] = has_ch ? cur[j].v[e] : (R)0;
                 }
                 const bool edge = x == 0 || x + V >= nx;
+                const bool keep = x <= 2 || x + V > nx - 3 || y < 3 || y >= ny - 3;
                 const R* er = rv + (2 * (y - y0) + (x == 0 ? 0 : 1)) * F;
                 group<R, V> c[F][NZ];
 #pragma unroll
@@ -532,8 +536,8 @@ __global__ void __launch_bounds__(rdt_threads(sizeof(R)) + 32, rdt_blocks(sizeof
                         group<R, V> w = gadd(c[f][z], evo[f]);
 #pragma unroll
                         for (int e = 0; e < V; ++e)
-                            if (edge && (x + e == 0 || x + e >= nx - 1)) w.v[e] = er[f];
-                        store_group(o + f * np + z * pxy, w);
+                            if (edge && (x + e == 0 || x + e >= nx - 1)) w.v[e] = carry ? c[f][z].v[e] : er[f];
+                        store_group(o + f * np + z * pxy, w, keep || (has_ch && z == 0));
                     }
                 }
             }
@@ -677,7 +681,6 @@ __global__ void __launch_bounds__(CY_THREADS + 32, cyt_blocks(sizeof(R), NI + NC
              const double* __restrict__ cin, int* __restrict__ err) {
     constexpr int CS = NI + NCP, px = (MC + V - 1) / V * V, npl = MC * px, PS = cyt_planes<sizeof(R)>();
     constexpr int nc = (MC * npl + 3) / 4 * 4;  // stored nodes of a species
-    constexpr uint32_t SPB = PS * npl * sizeof(R);  // bytes of a species in a stage
     extern __shared__ __align__(128) unsigned char rd_smem[];
     __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES];
     R* const ring = (R*)rd_smem;
@@ -818,261 +821,52 @@ __device__ __forceinline__ void block_sums(double (&v)[K], double* red) {
     }
 }
 
-// The Update of one site per block (CaSim/ParallelHybridSolver.cpp:159-175): mouth
-// values, Dirichlet rim from the cytosol, efflux through the rim, the RD3D deposits
-// into cytosol layer 0, RyR currents and the jSR coupling; the steps, their order and
-// the values they read are those of the generic k_update, the per-node quantities in
-// registers and the block sums by warp shuffles.
-template <typename R, int NI, int NP, bool RD3D>
-__global__ void __launch_bounds__(UP_THREADS) k_update_s(const __grid_constant__ cb_model m, int NS, const cb_site* __restrict__ sites,
-                                                         R* __restrict__ fld, R* __restrict__ curg, const int* __restrict__ ch_node,
-                                                         const int* __restrict__ ch_owner, const int* __restrict__ ch_state,
-                                                         double* __restrict__ mouth, cb_site_scalars* __restrict__ sc, int nc,
-                                                         const R* __restrict__ cyto, double* __restrict__ cin,
-                                                         const int* __restrict__ rim_cnode, const int* __restrict__ dep_ptr,
-                                                         const int* __restrict__ dep_term, const R* __restrict__ prev, int max_terms) {
-    constexpr int F = NI + NP;
-    constexpr int CSM = NI + 4;  // cytosol species slots (ions + at most 4 pairs)
-    const int CS = m.n_ions + m.c_n_pairs;
-    extern __shared__ double smem[];
-    double* red = smem;                   // (UP_THREADS / 32) * (F + NI)
-    double* terms = smem + 8 * (F + NI);  // RD3D: [term][F] efflux values
-    const int s = blockIdx.x;
-    const cb_site st = sites[s];
-    cb_site_scalars& q = sc[s];
-    R* u = fld + st.node_base * F;
-    const int nx = st.nx, ny = st.ny, nz = st.nz, px = st.px, nxy = px * ny;
-    const long long np = st.npad;
-    // RD3D: the site's deposit lists (per layer-0 cytosol node its efflux terms, in term
-    // order) staged in shared memory behind the terms, loaded here so that the loads
-    // overlap the phases before the deposit sums
-    const int zmax0 = nz == 1 ? 1 : nz - 1;
-    const int T0 = cb_efflux_terms(nx, ny, zmax0);
-    int* s_ptr = (int*)(terms + (size_t)max_terms * F);
-    int* s_term = s_ptr + (RD3D ? m.mc * m.mc + 1 : 0);
-    if (RD3D) {
-        const int mc2 = m.mc * m.mc;
-        const int* ptr = dep_ptr + (long long)s * (mc2 + 1);
-        for (int k = threadIdx.x; k <= mc2; k += UP_THREADS) s_ptr[k] = ptr[k];
-        const int* dtm = dep_term + st.term_off;
-        for (int k = threadIdx.x; k < T0; k += UP_THREADS) s_term[k] = dtm[k];
-    }
-    // 1. mouth values: ions, pairs, free buffers (CaSim/DyadRD2DCPU.cpp:361-380). After
-    // k_rd_v (prev set) the rim holds its Dirichlet values already; a RyR on the rim
-    // reads the value the step carried over there, which is prev's
-    for (int c = threadIdx.x; c < st.n_ch; c += UP_THREADS) {
-        const int node = ch_node[st.ch_off + c];
-        double* mo = mouth + (long long)(st.ch_off + c) * NS;
-        const R* src = u;
-        if (prev) {
-            const int cx = node % px, cyy = (node / px) % ny;
-            if (cx == 0 || cx == nx - 1 || cyy == 0 || cyy == ny - 1) src = prev + st.node_base * F;
-        }
-        double v[F];
-#pragma unroll
-        for (int f = 0; f < F; ++f) v[f] = (double)src[f * np + node];
-#pragma unroll
-        for (int f = 0; f < F; ++f) mo[f] = v[f];
-        for (int b = 0; b < m.n_buf; ++b) {
-            double fr = m.Ctot[b];
-#pragma unroll
-            for (int p = 0; p < NP; ++p)
-                if (m.pair_buf[p] == b) fr -= v[NI + p];
-            mo[F + b] = fr;
-        }
-    }
-    __syncthreads();
-    // 2. Dirichlet edges from the cytosol (CaSim/DyadRD2DCPU.cpp:274-303), unless k_rd_v
-    // set them (prev set)
-    const int nrim = prev ? 0 : cb_rim_count(nx, ny);
-    const R* cy = RD3D ? cyto + (long long)s * CS * nc : nullptr;
-    for (int t = threadIdx.x; t < nrim * nz; t += UP_THREADS) {
-        const int z = t / nrim, r = t - z * nrim;
-        int x, y;
-        cb_rim_xy(r, nx, ny, x, y);
-        const int node = x + px * y + nxy * z;
-        if (!RD3D) {
-#pragma unroll
-            for (int j = 0; j < NI; ++j) u[j * np + node] = (R)q.c_ions[j];
-#pragma unroll
-            for (int p = 0; p < NP; ++p) u[(NI + p) * np + node] = (R)q.c_bnd[p];
-        } else {
-            const int cn = rim_cnode[st.rim_off + r];
-#pragma unroll
-            for (int j = 0; j < NI; ++j) u[j * np + node] = cy[(long long)j * nc + cn];
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                const int cq = m.dyad_c_pair[p];
-                u[(NI + p) * np + node] = cq >= 0 ? cy[(long long)(NI + cq) * nc + cn] : (R)m.pair_init[p];
-            }
-        }
-    }
-    __syncthreads();
-    // 3. efflux (CaSim/DyadRD2DCPU.cpp:305-350): per-term values, block sums
-    const int zmax = nz == 1 ? 1 : nz - 1;
-    const int T = cb_efflux_terms(nx, ny, zmax);
-    double part[F];
-#pragma unroll
-    for (int f = 0; f < F; ++f) part[f] = 0;
-    for (int t = threadIdx.x; t < T; t += UP_THREADS) {
-        int x0, y0, x1, y1, x2, y2, z;
-        const int sel = cb_efflux_term(t, nx, ny, zmax, x0, y0, x1, y1, x2, y2, z);
-        const double sf = sel == 0 ? m.sx : m.sy;
-        const int n0 = x0 + px * y0 + nxy * z, n1 = x1 + px * y1 + nxy * z, n2 = x2 + px * y2 + nxy * z;
-        double a0[F], a1[F], a2[F];
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-            a0[f] = (double)u[f * np + n0];
-            a1[f] = (double)u[f * np + n1];
-            a2[f] = (double)u[f * np + n2];
-        }
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-            const double D = f < NI ? m.D_ion[f] : m.D_pair[f - NI];
-            const double g = 2 * a1[f] - 1.5 * a0[f] - 0.5 * a2[f];
-            if (!RD3D) {
-                part[f] += D * m.grad_mult * sf * g;
-            } else {
-                const double v = D * sf * g * m.inv_hc3;
-                part[f] += v;
-                terms[(long long)t * F + f] = v;
-            }
-        }
-    }
-    block_sums<F>(part, red);  // its barriers also publish the terms
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int f = 0; f < F; ++f) q.efflux[f] = part[f];
-    // 4. RD3D: deposit into the cytosol layer z = 0 in term order
-    if (RD3D) {
-        const int mc2 = m.mc * m.mc;
-        const int* ptr = s_ptr;
-        const int* dtm = s_term;
-        for (int cn = threadIdx.x; cn < mc2; cn += UP_THREADS) {
-            const int lo = ptr[cn], hi = ptr[cn + 1];
-            double acc[CSM];
-#pragma unroll
-            for (int c = 0; c < CSM; ++c) acc[c] = 0;
-            for (int k = lo; k < hi; ++k) {
-                const int t = dtm[k];
-#pragma unroll
-                for (int c = 0; c < CSM; ++c) {
-                    if (c >= CS) break;
-                    int f = c < NI ? c : m.c_dyad_pair[c - NI];
-                    if (f >= 0 && c >= NI) f += NI;
-                    if (f >= 0) acc[c] += terms[(long long)t * F + f];
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < CSM; ++c)
-                if (c < CS) cin[((long long)s * CS + c) * mc2 + cn] = acc[c];
-        }
-    }
-    // 5. RyR currents (CaSim/DyadRD2DCPU.cpp:243-264, CaSim/PassiveIonChannel.cpp:28-34)
-    R* cg = curg + st.node_base * NI;
-    double tot[NI];
-#pragma unroll
-    for (int j = 0; j < NI; ++j) tot[j] = 0;
-    for (int c = threadIdx.x; c < st.n_ch; c += UP_THREADS) {
-        const int node = ch_node[st.ch_off + c];
-        const int state = ch_state[st.ch_off + c];
-        const int own = ch_owner[st.ch_off + c];
-#pragma unroll
-        for (int j = 0; j < NI; ++j) {
-            const double flux = state * (m.g[j] * (q.jsr_new[j] - (double)u[j * np + node]));
-            if (own) cg[j * np + node] = (R)flux;
-            tot[j] += flux;
-        }
-    }
-    block_sums<NI>(tot, red);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int j = 0; j < NI; ++j) q.total[j] = tot[j];
-        // 6. jSR coupling (CaSim/SRPool.cpp:55-68)
-        if (!m.jsr_const)
-#pragma unroll
-            for (int i = 0; i < NI; ++i) {
-                q.IjSR[i] = q.total[i] * m.V_elem;
-                q.nsr[i] = m.nsr[i];
-                q.jsr[i] = q.jsr_new[i];
-            }
-    }
-}
-
-// Pools and two-state gating of one site per warp (CaSim/CytosolPool.cpp:217-268,
-// CaSim/SRPool.cpp:70-89, CaSim/DyadChannels.cpp:97-130). The site's MRG32k3a stream is
-// consumed in the reference's order (one draw per RyR test in RyR order, one more per
-// transition) without a serial loop: lane l jumps to draw l of the stream (jump table J,
-// row l: A^(2l)), the lanes draw 32 consecutive values at a time (then jump by A^62,
-// row 31, to their draw of the next 32), and 32 RyRs are resolved per ballot, one more
-// ballot after each transition. The stream state left behind is that at the first
-// unused draw, as after the serial loop. With site_gate set, site s gates by
-// gates[site_gate[s]] (per-site gating models) instead of the batch's model.
-// MWC60: the 60-state model (mwc.h): the lanes form 32 escape rates at a time, a
-// transition's second draw picks the micro-state it goes to (100 2D sites of 20 RyRs, FP64,
-// 200 steps and readback: 89.4 ms with a thread per site, 6.4 ms here).
-constexpr int PRE_WARPS = 4;
-template <bool MWC60>
-__global__ void __launch_bounds__(32 * PRE_WARPS) k_pre_r(const __grid_constant__ cb_model m, int S, int NS,
-                                                          const cb_site* __restrict__ sites, cb_site_scalars* __restrict__ sc,
-                                                          int* __restrict__ ch_state, const double* __restrict__ mouth,
-                                                          const double* __restrict__ spx0, const double* __restrict__ spc0,
-                                                          const double* __restrict__ spx1, const double* __restrict__ spc1,
-                                                          const unsigned long long* __restrict__ J, const cb_gate* __restrict__ gates,
-                                                          const int* __restrict__ site_gate, int* __restrict__ ch_micro,
-                                                          const cb_mwc_tab* __restrict__ mwc) {
-    __shared__ double s_u[PRE_WARPS][64];  // draws [we - 64, we), slot = draw & 63
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int s = blockIdx.x * PRE_WARPS + w;
-    if (s >= S) return;  // whole warp
-    const cb_site st = sites[s];
-    cb_site_scalars& q = sc[s];
-    const double dt = m.dt;
-    if (lane == 0) {
-        if (m.cyto_type == CB_CYTO_POOL) cb_pool_step(m, q, dt);
-        cb_jsr_step(m, q, dt);
-    }
+// RyR gating of one site by one warp (CaSim/DyadChannels.cpp:97-130), the transition
+// probabilities prob given. The site's MRG32k3a stream is consumed in the reference's order (one
+// draw per RyR test in RyR order, one more per transition) without a serial loop: lane l jumps
+// to draw l of the stream (jump table J, row l: A^(2l)), the lanes draw 32 consecutive values at
+// a time (then jump by A^62, row 31, to their draw of the next 32), and 32 RyRs are resolved per
+// ballot, one more ballot after each transition. The stream state left behind is that at the
+// first unused draw, as after the serial loop. (J is stored entry-major, [18][32 rows], so that the
+// lanes' rows load coalesced.) ring: 64 draws, [we - 64, we), slot = draw & 63.
+// The new open flags go to s_open as well. With mwc (60-state model) a transition's second draw
+// picks the micro-state, at the mouth concentrations pcm.
+__device__ __forceinline__ void gate_warp(const cb_site& st, cb_site_scalars& q, const double* __restrict__ prob, const double* __restrict__ pcm,
+                                          int* __restrict__ ch_state, int* __restrict__ ch_micro, const cb_mwc_tab* __restrict__ mwc,
+                                          const unsigned long long* __restrict__ J, double* ring, unsigned char* s_open) {
+    const int lane = threadIdx.x & 31;
     cbrng::State gl;  // this lane's draw we + lane
 #pragma unroll
     for (int i = 0; i < 6; ++i) gl.s[i] = q.rng[i];
-    cbrng::jump_by(J + 18 * lane, gl);
+    auto jump = [&](int row) {
+        unsigned long long a[18];
+#pragma unroll
+        for (int i = 0; i < 18; ++i) a[i] = J[32 * i + row];
+        cbrng::jump_by(a, gl);
+    };
+    jump(lane);
     cbrng::State gs = gl;  // state at this lane's draw of the latest chunk
     long long D = 0, we = 0;
-    const int nch = st.n_ch;
+    const int nch = st.n_ch, extra = mwc ? 1 : 0;
     for (int c0 = 0; c0 < nch; c0 += 32) {
         const int cnt = min(32, nch - c0);
         const int c = c0 + lane;
         const bool act = lane < cnt;
-        double p = 0, exit_rate = 0, ca = 0, mg = 0;
-        int stt = 0;
-        if (act) {
-            const double* mo = mouth + (long long)(st.ch_off + c) * NS;
-            ca = mo[m.ca_idx];
-            mg = m.mg_idx >= 0 ? mo[m.mg_idx] : 0.0;
-            stt = MWC60 ? ch_micro[st.ch_off + c] : ch_state[st.ch_off + c];
-            if (MWC60) {
-                exit_rate = cb_mwc_exit(*mwc, stt, ca, mg);
-                p = exit_rate * dt;
-            } else if (site_gate) {  // the site's own gating model
-                const cb_gate& g = gates[site_gate[s]];
-                p = cb_rate(g, g.spx[0], g.spc[0], g.spx[1], g.spc[1], stt, ca, mg) * dt;
-            } else {
-                p = cb_rate(m, spx0, spc0, spx1, spc1, stt, ca, mg) * dt;
-            }
-        }
+        const double p = act ? prob[st.ch_off + c] : 0.0;
+        int open = act ? ch_state[st.ch_off + c] : 0;
         int start = 0;
         while (start < cnt) {
-            // draws D .. D + (cnt - start) - 1 must be in the ring (MWC60: one more, the last
+            // draws D .. D + (cnt - start) - 1 must be in the ring (60-state: one more, the last
             // RyR's second draw; D + 33 at most, and chunks of 32 keep 64 draws)
-            while (we < D + (cnt - start) + (MWC60 ? 1 : 0)) {
+            while (we < D + (cnt - start) + extra) {
                 gs = gl;
-                s_u[w][(we + lane) & 63] = cbrng::u01d_fold(gl);
-                cbrng::jump_by(J + 18 * 31, gl);
+                ring[(we + lane) & 63] = cbrng::u01d_fold(gl);
+                jump(31);
                 we += 32;
                 __syncwarp();
             }
             const bool rem = act && lane >= start;
-            const double u = rem ? s_u[w][(D + (lane - start)) & 63] : 2.0;
+            const double u = rem ? ring[(D + (lane - start)) & 63] : 2.0;
             const unsigned int t = __ballot_sync(0xffffffffu, rem && (u < p));
             if (t == 0u) {
                 D += cnt - start;
@@ -1080,17 +874,21 @@ __global__ void __launch_bounds__(32 * PRE_WARPS) k_pre_r(const __grid_constant_
             }
             const int f = __ffs(t) - 1;
             if (lane == f) {
-                if (MWC60) {
-                    const int to = cb_mwc_next(*mwc, stt, ca, mg, exit_rate, s_u[w][(D + (f - start) + 1) & 63]);
+                if (mwc) {
+                    const int mi = ch_micro[st.ch_off + c];
+                    const double ca = pcm[2 * (st.ch_off + c)], mg = pcm[2 * (st.ch_off + c) + 1];
+                    const int to = cb_mwc_next(*mwc, mi, ca, mg, cb_mwc_exit(*mwc, mi, ca, mg), ring[(D + (f - start) + 1) & 63]);
                     ch_micro[st.ch_off + c] = to;
-                    ch_state[st.ch_off + c] = to >= CB_MWC_OPEN;
+                    open = to >= CB_MWC_OPEN;
                 } else {
-                    ch_state[st.ch_off + c] = 1 - stt;
+                    open = 1 - open;
                 }
+                ch_state[st.ch_off + c] = open;
             }
             D += (f - start) + 2;
             start = f + 1;
         }
+        if (act) s_open[c] = (unsigned char)open;
         __syncwarp();
     }
     // the state at draw D: lane D - (we - 32) of the latest chunk before its draw, or, past
@@ -1104,6 +902,346 @@ __global__ void __launch_bounds__(32 * PRE_WARPS) k_pre_r(const __grid_constant_
         q.draws += (unsigned long long)D;
 #pragma unroll
         for (int i = 0; i < 6; ++i) q.rng[i] = out[i];
+    }
+}
+
+// What the gating of the next step needs of RyR c: its transition probability at the mouth
+// concentrations (and, 60-state, the concentrations).
+struct gate_args {
+    const double *spx0, *spc0, *spx1, *spc1;
+    const unsigned long long* J;
+    const cb_gate* gates;      // per-site gating models, or null
+    const int* site_gate;
+    const cb_mwc_tab* mwc;     // 60-state model, or null
+    int* ch_state;
+    int* ch_micro;
+    double* prob;              // [RyR] scratch of one casim_b200_step call
+    double* pcm;               // [RyR][2]: mouth Ca and Mg (60-state)
+};
+__device__ __forceinline__ void store_prob(const cb_model& m, const gate_args& g, int s, int c, int open, double ca, double mg) {
+    double r;
+    if (g.mwc) {
+        r = cb_mwc_exit(*g.mwc, g.ch_micro[c], ca, mg);
+        g.pcm[2 * c] = ca;
+        g.pcm[2 * c + 1] = mg;
+    } else if (g.site_gate) {
+        const cb_gate& o = g.gates[g.site_gate[s]];
+        r = cb_rate(o, o.spx[0], o.spc[0], o.spx[1], o.spc[1], open, ca, mg);
+    } else {
+        r = cb_rate(m, g.spx0, g.spc0, g.spx1, g.spc1, open, ca, mg);
+    }
+    g.prob[c] = r * m.dt;
+}
+
+// the probabilities for the first step of a call, from the mouth values and RyR states as they are
+__global__ void k_prob(const __grid_constant__ cb_model m, const __grid_constant__ gate_args g, int NS, const cb_site* __restrict__ sites,
+                       const double* __restrict__ mouth) {
+    const cb_site st = sites[blockIdx.x];
+    for (int c = threadIdx.x; c < st.n_ch; c += blockDim.x) {
+        const double* mo = mouth + (long long)(st.ch_off + c) * NS;
+        store_prob(m, g, blockIdx.x, st.ch_off + c, g.ch_state[st.ch_off + c], mo[m.ca_idx], m.mg_idx >= 0 ? mo[m.mg_idx] : 0.0);
+    }
+}
+
+// RD3D deposits of a site: its efflux terms are stored grouped by receiving layer-0 cytosol
+// node; slot k feeds cytosol species c[k] from dyad species f[k]
+struct dep_args {
+    const int* pos;       // [term_off + term]: its place in the grouped order
+    const int* node_ptr;  // [site]: the first of its receiving nodes, [S]: their count
+    const int3* node;     // cytosol node (i + mc*j), first and end term
+    int max_nodes, n, f[MAX_F], c[MAX_F];
+};
+
+constexpr int CH_OWNER = 1, CH_RIM = 2;  // flags of a RyR beside its node: takes the node's flux; lies on the rim
+
+// One site per block. GATE (a time step): first the RyR gating (warp 0) and the pool ODEs (warp
+// 1), which nothing before them in the step needs, while the other warps form the efflux; then
+// the Update (CaSim/ParallelHybridSolver.cpp:159-175): mouth values, Dirichlet rim from the
+// cytosol (RD3D: k_rd_t set it), efflux through the rim, the RD3D deposits into cytosol layer 0,
+// RyR currents, the jSR coupling and the probabilities of the next gating. Without GATE (the
+// public Update) no time passes and the rim is always set here. want: also write what only
+// the getters read (mouth values, RD3D: efflux sums), for the last step of a call.
+//
+// The kernel is a chain of short latency-bound phases per site, so they overlap: gating in a
+// launch of its own took 18 us of a 64-site step and this kernel 21 us, most of it waiting; the
+// efflux indices took integer divisions, the deposits went through an index list, the RyRs'
+// nodes were fetched twice and the sums reduced twice.
+template <typename R, int NI, int NP, bool RD3D, bool GATE>
+__global__ void __launch_bounds__(UP_THREADS, 4)
+    k_update_s(const __grid_constant__ cb_model m, const __grid_constant__ gate_args ga, const __grid_constant__ dep_args dep, int NS, bool want,
+               const cb_site* __restrict__ sites, R* __restrict__ fld, const R* __restrict__ prev, R* __restrict__ curg,
+               const int2* __restrict__ ch, double* __restrict__ mouth, cb_site_scalars* __restrict__ sc,
+               int nc, const R* __restrict__ cyto, double* __restrict__ cin, const int* __restrict__ rim_cnode, int max_ch, int max_terms) {
+    constexpr int F = NI + NP;
+    extern __shared__ double up_smem[];
+    __shared__ double red[UP_THREADS / 32 * (F + NI)], s_ring[64], s_jsr[NI];
+    __shared__ R s_rim[F];
+    unsigned char* s_open = (unsigned char*)up_smem;                    // [max_ch]
+    double* terms = up_smem + (max_ch + 7) / 8;                         // RD3D: [dep.n][max_terms]
+    int3* s_node = (int3*)(terms + (RD3D ? dep.n * max_terms : 0));     // RD3D: [dep.max_nodes]
+    const int s = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const cb_site st = sites[s];
+    cb_site_scalars& q = sc[s];
+    R* u = fld + st.node_base * F;
+    const R* before = GATE ? prev + st.node_base * F : u;
+    const int nx = st.nx, ny = st.ny, nz = st.nz, px = st.px, nxy = px * ny, np = st.npad;
+    const int2* chs = ch + st.ch_off;
+    // the warps of the efflux: all, or those that neither gate nor (RD3D) step the jSR
+    constexpr int E0 = !GATE ? 0 : RD3D ? 64 : 32, EN = UP_THREADS - E0;
+    const int et = tid - E0;
+    // 1. mouth values: ions, pairs, free buffers (CaSim/DyadRD2DCPU.cpp:361-380): the new fields, a
+    // RyR on the rim what the step carried over there, which is before's (GATE: the rim is set
+    // already or set below). Each thread keeps its first RyR's.
+    int2 ch0 = make_int2(0, 0);
+    R v0[F];
+    for (int c = tid; c < st.n_ch; c += UP_THREADS) {
+        const int2 cc = chs[c];
+        const R* src = cc.y & CH_RIM ? before : u;
+        R v[F];
+#pragma unroll
+        for (int f = 0; f < F; ++f) v[f] = src[f * np + cc.x];
+        if (c == tid) {
+            ch0 = cc;
+#pragma unroll
+            for (int f = 0; f < F; ++f) v0[f] = v[f];
+        }
+        if (!want) break;
+        double* mo = mouth + (long long)(st.ch_off + c) * NS;
+#pragma unroll
+        for (int f = 0; f < F; ++f) mo[f] = (double)v[f];
+        for (int b = 0; b < m.n_buf; ++b) {
+            double fr = m.Ctot[b];
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                if (m.pair_buf[p] == b) fr -= (double)v[NI + p];
+            mo[F + b] = fr;
+        }
+    }
+    auto efflux_sync = [&]() {
+        if (GATE) {
+            __syncwarp();
+            asm volatile("bar.sync 1, %0;" ::"n"(EN) : "memory");
+        } else {
+            __syncthreads();
+        }
+    };
+    double part[F];
+#pragma unroll
+    for (int f = 0; f < F; ++f) part[f] = 0;
+    if (GATE && warp == 0) {
+        gate_warp(st, q, ga.prob, ga.pcm, ga.ch_state, ga.ch_micro, ga.mwc, ga.J, s_ring, s_open);
+    } else if (GATE && RD3D && warp == 1) {
+        if (lane == 0) {
+            cb_jsr_step(m, q, m.dt);
+#pragma unroll
+            for (int j = 0; j < NI; ++j) s_jsr[j] = q.jsr_new[j];
+        }
+    } else {
+        if (et == 0) {
+            if (GATE && !RD3D) cb_pool_step(m, q, m.dt);
+#pragma unroll
+            for (int j = 0; j < NI; ++j) s_rim[j] = (R)q.c_ions[j];
+#pragma unroll
+            for (int p = 0; p < NP; ++p) s_rim[NI + p] = (R)q.c_bnd[p];
+        }
+        __syncwarp();
+        // RD3D: the site's deposit nodes, staged while the efflux loads are in flight
+        int nd = 0;
+        if (RD3D) {
+            const int d0 = dep.node_ptr[s];
+            nd = dep.node_ptr[s + 1] - d0;
+            for (int i = et; i < nd; i += EN) s_node[i] = dep.node[d0 + i];
+        }
+        // 2. Dirichlet edges from the cytosol (CaSim/DyadRD2DCPU.cpp:274-303)
+        auto set_rim = [&]() {
+            const int nrim = cb_rim_count(nx, ny);
+            const R* cy = RD3D ? cyto + (long long)s * (m.n_ions + m.c_n_pairs) * nc : nullptr;
+            for (int r = et; r < nrim; r += EN) {
+                int x, y;
+                cb_rim_xy(r, nx, ny, x, y);
+                R b[F];
+                if (!RD3D) {
+#pragma unroll
+                    for (int f = 0; f < F; ++f) b[f] = s_rim[f];
+                } else {
+                    const int cn = rim_cnode[st.rim_off + r];
+#pragma unroll
+                    for (int j = 0; j < NI; ++j) b[j] = cy[j * nc + cn];
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        const int cq = m.dyad_c_pair[p];
+                        b[NI + p] = cq >= 0 ? cy[(NI + cq) * nc + cn] : (R)m.pair_init[p];
+                    }
+                }
+                for (int z = 0; z < nz; ++z)
+#pragma unroll
+                    for (int f = 0; f < F; ++f) u[f * np + x + px * y + nxy * z] = b[f];
+            }
+        };
+        if (!GATE) {
+            efflux_sync();
+            set_rim();
+            efflux_sync();
+        }
+        // 3. efflux (CaSim/DyadRD2DCPU.cpp:305-350) in the reference's term order: x-edges (x = 0,
+        // then nx-1) over y = 1..ny-2, y-edges over x, layers innermost (the top one has no rim).
+        // A thread's NB terms are loaded together. Pool, GATE: the rim nodes read s_rim.
+        constexpr int NB = 2;
+        constexpr bool POOL = GATE && !RD3D;
+        const int zs = nz == 1 ? 0 : 1, nye = ny - 2, T = (2 * nye + 2 * nx) << zs;
+        const int* pos = RD3D ? dep.pos + st.term_off : nullptr;
+        bool synced = !POOL;
+        for (int t0 = et; t0 < T || !synced; t0 += NB * EN) {
+            R a0[NB][F], a1[NB][F], a2[NB][F];
+            int at[NB];
+            double sf[NB];
+            bool end[NB];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const int t = t0 + i * EN;
+                if (t >= T) break;
+                const int z = zs ? t & 1 : 0;
+                int a = t >> zs, n0, step;
+                const bool xe = a < 2 * nye;
+                if (xe) {
+                    const bool far = a >= nye;
+                    n0 = px * (1 + a - (far ? nye : 0)) + (far ? nx - 1 : 0);
+                    step = far ? -1 : 1;
+                    end[i] = false;
+                } else {
+                    a -= 2 * nye;
+                    const bool far = a >= nx;
+                    a -= far ? nx : 0;
+                    n0 = a + (far ? px * (ny - 1) : 0);
+                    step = far ? -px : px;
+                    end[i] = a == 0 || a == nx - 1;  // the line runs along the rim
+                }
+                n0 += nxy * z;
+                sf[i] = xe ? m.sx : m.sy;
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    if (!POOL) a0[i][f] = u[f * np + n0];
+                    a1[i][f] = u[f * np + n0 + step];
+                    a2[i][f] = u[f * np + n0 + 2 * step];
+                }
+                at[i] = RD3D ? pos[t] : 0;
+            }
+            if (!synced) {  // the pool's new values
+                efflux_sync();
+                synced = true;
+            }
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                if (t0 + i * EN >= T) break;
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    if (POOL) {
+                        a0[i][f] = s_rim[f];
+                        if (end[i]) a1[i][f] = a2[i][f] = s_rim[f];
+                    }
+                    const double D = f < NI ? m.D_ion[f] : m.D_pair[f - NI];
+                    const double g = 2 * (double)a1[i][f] - 1.5 * (double)a0[i][f] - 0.5 * (double)a2[i][f];
+                    if (!RD3D) {
+                        part[f] += D * m.grad_mult * sf[i] * g;
+                    } else {
+                        const double v = D * sf[i] * g * m.inv_hc3;
+                        part[f] += v;
+#pragma unroll
+                        for (int k = 0; k < F; ++k)
+                            if (k < dep.n && dep.f[k] == f) terms[k * max_terms + at[i]] = v;
+                    }
+                }
+            }
+        }
+        if (POOL) {
+            set_rim();
+            if (et == 0) {
+                cb_jsr_step(m, q, m.dt);
+            }
+        }
+        if (!RD3D || !GATE) {
+            if (et == 0)
+#pragma unroll
+                for (int j = 0; j < NI; ++j) s_jsr[j] = q.jsr_new[j];
+        }
+        // 4. RD3D: deposits into the cytosol layer z = 0 (the other nodes' deposits stay zero): 8
+        // lanes per receiving node, every 8th of its terms each (most nodes have 8, those under
+        // the corners of a cleft wider than the cytosol dozens)
+        if (RD3D) {
+            efflux_sync();
+            const int mc2 = m.mc * m.mc;
+            for (int i = et >> 3; i < (nd + EN / 8 - 1) / (EN / 8) * (EN / 8); i += EN / 8) {
+                const int3 dn = i < nd ? s_node[i] : make_int3(0, 0, 0);
+                double acc[F];
+#pragma unroll
+                for (int k = 0; k < F; ++k) acc[k] = 0;
+                for (int t = dn.y + (lane & 7); t < dn.z; t += 8)
+#pragma unroll
+                    for (int k = 0; k < F; ++k)
+                        if (k < dep.n) acc[k] += terms[k * max_terms + t];
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                    for (int k = 0; k < F; ++k)
+                        if (k < dep.n) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+                if (i < nd && (lane & 7) == 0)
+#pragma unroll
+                    for (int k = 0; k < F; ++k)
+                        if (k < dep.n) cin[((long long)s * (m.n_ions + m.c_n_pairs) + dep.c[k]) * mc2 + dn.x] = acc[k];
+            }
+        }
+    }
+    __syncthreads();
+    // 5. RyR currents (CaSim/DyadRD2DCPU.cpp:243-264, CaSim/PassiveIonChannel.cpp:28-34) and the
+    // next gating's probabilities
+    R* cg = curg + st.node_base * NI;
+    double sums[F + NI];
+#pragma unroll
+    for (int f = 0; f < F; ++f) sums[f] = part[f];
+#pragma unroll
+    for (int j = 0; j < NI; ++j) sums[F + j] = 0;
+    for (int c = tid; c < st.n_ch; c += UP_THREADS) {
+        const int2 cc = c == tid ? ch0 : chs[c];
+        const int open = GATE ? (int)s_open[c] : ga.ch_state[st.ch_off + c];
+        const R* src = cc.y & CH_RIM ? before : u;
+        double ca = 0, mg = 0;
+#pragma unroll
+        for (int j = 0; j < NI; ++j) {
+            const R mv = c == tid ? v0[j] : src[j * np + cc.x];
+            // the flux reads the node after the rim is set
+            const R at = !(cc.y & CH_RIM) ? mv : GATE && !RD3D ? s_rim[j] : u[j * np + cc.x];
+            const double flux = open * (m.g[j] * (s_jsr[j] - (double)at));
+            if (cc.y & CH_OWNER) cg[j * np + cc.x] = (R)flux;
+            sums[F + j] += flux;
+            if (j == m.ca_idx) ca = (double)mv;
+            if (j == m.mg_idx) mg = (double)mv;
+        }
+        if (GATE) store_prob(m, ga, s, st.ch_off + c, open, ca, mg);
+    }
+    if (!RD3D || !GATE || want) {
+        block_sums<F + NI>(sums, red);
+    } else {
+        double tot[NI];
+#pragma unroll
+        for (int j = 0; j < NI; ++j) tot[j] = sums[F + j];
+        block_sums<NI>(tot, red);
+#pragma unroll
+        for (int j = 0; j < NI; ++j) sums[F + j] = tot[j];
+    }
+    if (tid == 0) {
+        if (!RD3D || !GATE || want)
+#pragma unroll
+            for (int f = 0; f < F; ++f) q.efflux[f] = sums[f];
+#pragma unroll
+        for (int j = 0; j < NI; ++j) q.total[j] = sums[F + j];
+        // 6. jSR coupling (CaSim/SRPool.cpp:55-68)
+        if (!m.jsr_const)
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                q.IjSR[i] = sums[F + i] * m.V_elem;
+                q.nsr[i] = m.nsr[i];
+                q.jsr[i] = s_jsr[i];
+            }
     }
 }
 
