@@ -44,6 +44,7 @@ struct cb_dev {
     // spline tables
     double* spx[2] = {nullptr, nullptr};
     double* spc[2] = {nullptr, nullptr};
+    double* gathered = nullptr;       // [ch] one species of mouth, for the batch getter; first use
     // bookkeeping
     int* err_host = nullptr;          // set to 1 by a kernel whose bounded wait ran out (mapped host memory)
     int* err_flag = nullptr;          // its device address
@@ -87,6 +88,9 @@ bool cb_plain_streaming(cb_dev& d);
 bool cb_plain_gating_ready(cb_dev& d);
 // one plain time step with ev[0..4] recorded around its four kernels
 cudaError_t cb_plain_step_marked(cb_dev& d, cudaStream_t st, cudaEvent_t* ev);
+
+// one species' mouth values of every RyR side by side (plain.cu)
+cudaError_t cb_gather_mouth(const cb_dev& d, int species, double* out, cudaStream_t st);
 
 // surrogate-driven gating without the RD step (plain.cu)
 cudaError_t cb_sg_features(cb_dev& d, int max_ch, int ld, float* X, cudaStream_t st);

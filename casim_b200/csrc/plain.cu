@@ -966,6 +966,18 @@ cudaError_t cb_plain_step(cb_dev& d, long long n, cudaStream_t st, long long* la
     return cudaSuccess;
 }
 
+namespace {
+__global__ void k_gather_mouth(long long n, int NS, int species, const double* __restrict__ mouth, double* __restrict__ out) {
+    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (c < n) out[c] = mouth[c * NS + species];
+}
+}  // namespace
+
+cudaError_t cb_gather_mouth(const cb_dev& d, int species, double* out, cudaStream_t st) {
+    k_gather_mouth<<<(unsigned)((d.total_ch + 255) / 256), 256, 0, st>>>(d.total_ch, d.NS, species, d.mouth, out);
+    return cudaGetLastError();
+}
+
 cudaError_t cb_sg_features(cb_dev& d, int max_ch, int ld, float* X, cudaStream_t st) {
     k_sg_features<<<(d.S + 127) / 128, 128, 0, st>>>(d.S, d.m.n_buf, max_ch, ld, d.sites, d.ch_node, d.ch_state, d.sc, X);
     return cudaGetLastError();
