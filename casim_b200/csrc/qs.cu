@@ -256,7 +256,7 @@ __host__ __device__ inline size_t qs_added_bytes(int n_ch) { return n_ch <= 64 ?
 
 // Scenarios on persistent warps (CaSim/QuasyStationaryReleaseSite.cpp:89-133). 4096 scenarios of a
 // 48-RyR MWC site, run and analysis: 2.60 ms with lane 0 summing the rates and walking the shares,
-// 1.31 ms by scans over the lanes.
+// 2.02 ms by scans over the lanes.
 template <int MODEL>
 __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, const double* __restrict__ added, double bg, double mg,
                                                           double max_time, int n_scen, const int* __restrict__ first,

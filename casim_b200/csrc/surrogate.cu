@@ -42,6 +42,7 @@ struct gemm_args {
     const bf16* B;  // [N][K]
     int M, N, K;
     int BN;         // columns per CTA (grid.y = N / BN)
+    int kz;         // K of one slice; slice z (grid.z) writes C + z * M * N (EPI_PLAIN), 0: all of K
     int mode;
     const float* bias;  // [N]
     float* C;           // [M][N] FP32 (EPI_OUT, EPI_PLAIN)
@@ -145,10 +146,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(const __grid_constant__ gem
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const uint32_t idesc = idesc_bf16(g.BN);
-    const int kt = g.K / BK;
+    const int kz = g.kz > 0 ? g.kz : g.K, kbase = blockIdx.z * kz;
+    const int kt = min(kz, g.K - kbase) / BK;
     bool ok = true;
 
-    load_stage(g, m0, n0, 0, sa[0], sb[0]);
+    load_stage(g, m0, n0, kbase, sa[0], sb[0]);
     for (int i = 0; i < kt; ++i) {
         const int s = i & 1;
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(const __grid_constant__ gem
         if (i + 1 < kt) {
             const int s2 = (i + 1) & 1;
             if (i >= 1) ok = mbar_wait(&bars[s2], (uint32_t)(((i - 1) >> 1) & 1)) && ok;  // slice i-1 consumed
-            load_stage(g, m0, n0, (i + 1) * BK, sa[s2], sb[s2]);
+            load_stage(g, m0, n0, kbase + (i + 1) * BK, sa[s2], sb[s2]);
         }
     }
     ok = mbar_wait(&bars[(kt - 1) & 1], (uint32_t)(((kt - 1) >> 1) & 1)) && ok;
@@ -187,25 +189,31 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(const __grid_constant__ gem
         const int cg = n0 + c0;  // global column
         const size_t o = (size_t)row * g.N + cg;
         if (g.mode == EPI_PLAIN) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) g.C[o + j] = v[j];
+            float4* c = (float4*)(g.C + (size_t)blockIdx.z * g.M * g.N + o);
+            c[0] = make_float4(v[0], v[1], v[2], v[3]);
+            c[1] = make_float4(v[4], v[5], v[6], v[7]);
         } else if (g.mode == EPI_OUT) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) g.C[o + j] = v[j] + g.bias[cg + j];
         } else {
             __align__(16) bf16 h[8];
+            float4* zp = (float4*)(g.Z + o);
+            float z[8];
+            if (g.mode == EPI_HIDDEN) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float y;
-                if (g.mode == EPI_HIDDEN) {
-                    const float z = v[j] + g.bias[cg + j];
-                    if (g.Z) g.Z[o + j] = z;
-                    y = gelu(z);
-                } else {  // EPI_BACK: gradient w.r.t. the pre-activation
-                    y = v[j] * gelu_grad(g.Z[o + j]);
+                for (int j = 0; j < 8; ++j) z[j] = v[j] + g.bias[cg + j];
+                if (g.Z) {
+                    zp[0] = make_float4(z[0], z[1], z[2], z[3]);
+                    zp[1] = make_float4(z[4], z[5], z[6], z[7]);
                 }
-                h[j] = __float2bfloat16_rn(y);
+            } else {
+                const float4 p = zp[0], q = zp[1];
+                z[0] = p.x, z[1] = p.y, z[2] = p.z, z[3] = p.w;
+                z[4] = q.x, z[5] = q.y, z[6] = q.z, z[7] = q.w;
             }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)  // EPI_BACK: gradient w.r.t. the pre-activation
+                h[j] = __float2bfloat16_rn(g.mode == EPI_HIDDEN ? gelu(z[j]) : v[j] * gelu_grad(z[j]));
             *(uint4*)(g.H + o) = *(const uint4*)h;
             if (g.HT)
 #pragma unroll
@@ -269,34 +277,75 @@ __global__ void k_sum(const float* __restrict__ partial, int n, float scale, flo
     if (threadIdx.x == 0) *out = red[0] * scale;
 }
 
-// bias gradient: row sums of dZ^T [N][B], one warp per row, fixed order
+// bias gradient: row sums of dZ^T [N][B], one warp per row, 16-byte loads (B is a multiple of
+// 128), fixed order
 __global__ void k_rowsum(const bf16* __restrict__ dzt, int N, int B, float* __restrict__ db) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= N) return;
     float s = 0;
-    for (int i = lane; i < B; i += 32) s += __bfloat162float(dzt[(size_t)w * B + i]);
+    const uint4* row = (const uint4*)(dzt + (size_t)w * B);
+#pragma unroll 4
+    for (int i = lane; i < B / 8; i += 32) {
+        const uint4 q = row[i];
+        const __nv_bfloat162* h = (const __nv_bfloat162*)&q;
+        float2 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) t[j] = __bfloat1622float2(h[j]);
+        s += ((t[0].x + t[0].y) + (t[1].x + t[1].y)) + ((t[2].x + t[2].y) + (t[3].x + t[3].y));
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) db[w] = s;
 }
 
-// Adam on FP32 master weights [N][K] (+ bias [N]); BF16 copies W [N][K] and W^T [K][N]
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g, int N, int K,
-                       float lr, float b1, float b2, float eps, float c1, float c2, bf16* __restrict__ wb, bf16* __restrict__ wt) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= (long long)N * K) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1 - b1) * gi;
-    const float vi = b2 * v[i] + (1 - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) {
-        const int r = (int)(i / K), c = (int)(i - (long long)r * K);
-        const bf16 b = __float2bfloat16_rn(wi);
-        wb[i] = b;
-        wt[(size_t)c * N + r] = b;
+// A layer's tensors for the kernels that take all layers in one launch (grid.y: layer).
+constexpr int LAYERS = 16;  // layers per launch
+struct layer_set {
+    struct {
+        int N, K, splits;
+        float *w, *m, *v, *b, *mb, *vb;  // FP32 master weights [N][K], biases [N], their moments
+        float *dw, *db;                  // gradients
+        const float* part;               // [splits][N][K]: partial weight gradients
+        bf16 *wb, *wt;                   // BF16 copies W [N][K] and W^T [K][N]
+    } l[LAYERS];
+};
+
+// weight gradients: the sums of their K slices in slice order
+__global__ void k_grad_sum(const __grid_constant__ layer_set s) {
+    const auto& l = s.l[blockIdx.y];
+    const int n4 = l.N * l.K / 4;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
+        float4 a = ((const float4*)l.part)[i];
+#pragma unroll 4
+        for (int z = 1; z < l.splits; ++z) {
+            const float4 p = ((const float4*)l.part)[(size_t)z * n4 + i];
+            a.x += p.x, a.y += p.y, a.z += p.z, a.w += p.w;
+        }
+        ((float4*)l.dw)[i] = a;
+    }
+}
+
+// Adam on all layers' weights and biases; BF16 copies of the weights
+__global__ void k_adam(const __grid_constant__ layer_set s, float lr, float b1, float b2, float eps, float c1, float c2) {
+    const auto& l = s.l[blockIdx.y];
+    const int nw = l.N * l.K;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw + l.N; i += gridDim.x * blockDim.x) {
+        const bool bias = i >= nw;
+        const int k = bias ? i - nw : i;
+        float *w = bias ? l.b : l.w, *m = bias ? l.mb : l.m, *v = bias ? l.vb : l.v;
+        const float gi = (bias ? l.db : l.dw)[k];
+        const float mi = b1 * m[k] + (1 - b1) * gi;
+        const float vi = b2 * v[k] + (1 - b2) * gi * gi;
+        m[k] = mi;
+        v[k] = vi;
+        const float wi = w[k] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        w[k] = wi;
+        if (!bias) {
+            const int r = k / l.K, c = k - r * l.K;
+            const bf16 b = __float2bfloat16_rn(wi);
+            l.wb[k] = b;
+            l.wt[(size_t)c * l.N + r] = b;
+        }
     }
 }
 
@@ -325,6 +374,7 @@ struct casim_surrogate_s {
     float* Y = nullptr;                                  // [cap][out_pad]
     bf16 *DZ[2] = {nullptr, nullptr}, *DZT[2] = {nullptr, nullptr};
     float* partial = nullptr;
+    std::vector<float*> dWp;                             // [splits][dout][din]: K slices of the weight gradients
     float* loss = nullptr;
     int* err = nullptr;
     long long step = 0;
@@ -371,7 +421,7 @@ cudaError_t gemm(casim_sg h, gemm_args g) {
         if (e != cudaSuccess) return e;
         h->smem_max = sm;
     }
-    k_gemm<<<dim3(g.M / BM, g.N / g.BN), THREADS, sm, h->stream>>>(g);
+    k_gemm<<<dim3(g.M / BM, g.N / g.BN, g.kz > 0 ? (g.K + g.kz - 1) / g.kz : 1), THREADS, sm, h->stream>>>(g);
     h->launches++;
     return cudaGetLastError();
 }
@@ -382,6 +432,16 @@ unsigned long long splitmix(unsigned long long& s) {
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
     return z ^ (z >> 31);
 }
+
+// K slices of a weight gradient [N][K] over a batch of B rows: with one CTA per tile and all of B
+// in sequence, the four tiles of a 256 x 256 layer walked 64 slices each, two thirds of a training
+// step of 4096 rows. About one tile-slice per SM, at least 128 rows each (1060 us per step -> 240).
+int slice_of(int N, int K, int B) {
+    const int tiles = N / BM * (K / tile_n(K));
+    const int want = (int)(((long long)B * tiles / 148 + BK - 1) / BK * BK);
+    return std::min(B, std::max(2 * BK, want));
+}
+int slices(int kz, int B) { return (B + kz - 1) / kz; }
 
 cudaError_t ensure_capacity(casim_sg h, int B) {
     if (B <= h->cap) return cudaSuccess;
@@ -400,6 +460,8 @@ cudaError_t ensure_capacity(casim_sg h, int B) {
         fr(h->DZT[i]);
     }
     fr(h->partial);
+    for (auto p : h->dWp) fr(p);
+    h->dWp.assign(h->L, nullptr);
     int maxw = std::max(h->width, h->out_pad);
     h->Z.assign(h->L, nullptr);
     h->Hb.assign(h->L, nullptr);
@@ -450,9 +512,45 @@ cudaError_t forward(casim_sg h, const float* x, int B, bool train) {
     return cudaSuccess;
 }
 
+layer_set layers_from(casim_sg h, int l0, int B) {
+    layer_set s{};
+    for (int l = l0; l < std::min(h->L, l0 + LAYERS); ++l) {
+        auto& o = s.l[l - l0];
+        o.N = h->dout[l];
+        o.K = h->din[l];
+        o.splits = slices(slice_of(o.N, o.K, B), B);
+        o.w = h->W[l];
+        o.m = h->mW[l];
+        o.v = h->vW[l];
+        o.b = h->b[l];
+        o.mb = h->mb[l];
+        o.vb = h->vb[l];
+        o.dw = h->dW[l];
+        o.db = h->db[l];
+        o.part = h->dWp[l];
+        o.wb = h->Wb[l];
+        o.wt = h->WTb[l];
+    }
+    return s;
+}
+
+// the slices' workspaces, sized for the largest batch so far (a smaller one has no more slices than
+// tiles fill the chip: the slice count is bounded by B / 128)
+cudaError_t ensure_slices(casim_sg h) {
+    for (int l = 0; l < h->L; ++l)
+        if (!h->dWp[l]) {
+            int most = 1;
+            for (int b = BM; b <= h->cap; b += BM) most = std::max(most, slices(slice_of(h->dout[l], h->din[l], b), b));
+            const cudaError_t e = dalloc(&h->dWp[l], (size_t)most * h->dout[l] * h->din[l]);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
 // loss and gradients of all parameters into dW / db
 cudaError_t backward(casim_sg h, const float* t, int B) {
     cudaError_t e;
+    if ((e = ensure_slices(h)) != cudaSuccess) return e;
     const long long ny = (long long)B * h->out_pad;
     const int nb = (int)((ny + 255) / 256);
     k_mse<<<nb, 256, 0, h->stream>>>(h->Y, h->out_pad, t, B, h->n_out, h->DZ[0], h->DZT[0], h->partial);
@@ -467,7 +565,8 @@ cudaError_t backward(casim_sg h, const float* t, int B) {
         g.N = h->din[l];
         g.K = B;
         g.mode = EPI_PLAIN;
-        g.C = h->dW[l];
+        g.C = h->dWp[l];
+        g.kz = slice_of(g.M, g.N, B);
         g.err = h->err;
         if ((e = gemm(h, g)) != cudaSuccess) return e;
         k_rowsum<<<(h->dout[l] * 32 + 255) / 256, 256, 0, h->stream>>>(h->DZT[cur], h->dout[l], B, h->db[l]);
@@ -488,7 +587,11 @@ cudaError_t backward(casim_sg h, const float* t, int B) {
             cur ^= 1;
         }
     }
-    return cudaSuccess;
+    for (int l0 = 0; l0 < h->L; l0 += LAYERS) {
+        k_grad_sum<<<dim3(64, std::min(LAYERS, h->L - l0)), 256, 0, h->stream>>>(layers_from(h, l0, B));
+        h->launches++;
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t check_err(casim_sg h) {
@@ -617,6 +720,7 @@ casim_status casim_b200_sg_destroy(casim_sg h) {
         fr(h->DZT[i]);
     }
     fr(h->partial);
+    for (float* p : h->dWp) fr(p);
     fr(h->loss);
     fr(h->err);
     delete h;
@@ -697,15 +801,11 @@ casim_status casim_b200_sg_train_step(casim_sg h, const float* x_dev, const floa
         h->step++;
         const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
         const float c1 = 1.0f - (float)std::pow(b1, (double)h->step), c2 = 1.0f - (float)std::pow(b2, (double)h->step);
-        for (int l = 0; l < h->L && e == cudaSuccess; ++l) {
-            const int N = h->dout[l], K = h->din[l];
-            k_adam<<<(N * K + 255) / 256, 256, 0, h->stream>>>(h->W[l], h->mW[l], h->vW[l], h->dW[l], N, K, lr, b1, b2, eps, c1, c2,
-                                                             h->Wb[l], h->WTb[l]);
-            k_adam<<<(N + 255) / 256, 256, 0, h->stream>>>(h->b[l], h->mb[l], h->vb[l], h->db[l], N, 1, lr, b1, b2, eps, c1, c2,
-                                                         nullptr, nullptr);
-            h->launches += 2;
-            e = cudaGetLastError();
+        for (int l0 = 0; l0 < h->L; l0 += LAYERS) {
+            k_adam<<<dim3(128, std::min(LAYERS, h->L - l0)), 256, 0, h->stream>>>(layers_from(h, l0, batch), lr, b1, b2, eps, c1, c2);
+            h->launches++;
         }
+        e = cudaGetLastError();
     }
     if (e == cudaSuccess && loss) {
         e = cudaMemcpyAsync(loss, h->loss, 4, cudaMemcpyDeviceToHost, h->stream);
