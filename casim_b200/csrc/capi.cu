@@ -17,6 +17,30 @@
 #include "mrg32k3a.cuh"
 #include "physics.cuh"
 
+// Error words that kernels with bounded waits set, in mapped host memory so that a check costs no
+// copy. Page-locking takes milliseconds, so handles share pages of words: each takes a free one and
+// gives it back; a page is allocated when all words of the earlier ones are taken.
+namespace {
+std::mutex g_flag_lock;
+std::vector<int*> g_flags;
+}  // namespace
+int* cb_take_flag() {
+    std::lock_guard<std::mutex> g(g_flag_lock);
+    if (g_flags.empty()) {
+        int* p = nullptr;
+        if (cudaHostAlloc((void**)&p, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        for (int i = 0; i < 1024; ++i) g_flags.push_back(p + i);
+    }
+    int* f = g_flags.back();
+    g_flags.pop_back();
+    *f = 0;
+    return f;
+}
+void cb_give_flag(int* f) {
+    std::lock_guard<std::mutex> g(g_flag_lock);
+    g_flags.push_back(f);
+}
+
 struct casim_b200_sim {
     cb_config cfg;
     cb_dev d;
@@ -97,28 +121,6 @@ casim_status set_err(casim_b200_sim* h, casim_status s, const std::string& msg) 
     catch (const std::exception& e) {                                       \
         return set_err(h, CASIM_EINVAL, e.what());                          \
     }
-
-// Error words that kernels with bounded waits set, in mapped host memory so that a check costs no
-// copy. Page-locking takes milliseconds, so handles share pages of words: each takes a free one and
-// gives it back; a page is allocated when all words of the earlier ones are taken.
-std::mutex g_flag_lock;
-std::vector<int*> g_flags;
-int* take_flag() {
-    std::lock_guard<std::mutex> g(g_flag_lock);
-    if (g_flags.empty()) {
-        int* p = nullptr;
-        ck(cudaHostAlloc((void**)&p, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
-        for (int i = 0; i < 1024; ++i) g_flags.push_back(p + i);
-    }
-    int* f = g_flags.back();
-    g_flags.pop_back();
-    *f = 0;
-    return f;
-}
-void give_flag(int* f) {
-    std::lock_guard<std::mutex> g(g_flag_lock);
-    g_flags.push_back(f);
-}
 
 // a kernel's bounded wait for its own copies ran out in an earlier launch (the state is not valid)
 bool wait_gave_up(casim_b200_sim* h) {
@@ -267,7 +269,8 @@ void build_device(casim_b200_sim* h, int precision) {
             d.spx[w] = dupload(h, cfg.sp_x[w]);
             d.spc[w] = dupload(h, cfg.sp_c[w]);
         }
-    d.err_host = take_flag();
+    d.err_host = cb_take_flag();
+    if (!d.err_host) throw cuda_fail(cudaErrorMemoryAllocation, "cudaHostAlloc");
     ck(cudaHostGetDevicePointer((void**)&d.err_flag, d.err_host, 0), "cudaHostGetDevicePointer");
 }
 
@@ -353,7 +356,7 @@ casim_status casim_b200_destroy(casim_h h) {
     if (h->d.st_tiles) cudaFree(h->d.st_tiles);
     for (void* p : {h->d.st_runs, (void*)h->d.st_prob, (void*)h->d.st_ch})
         if (p) cudaFree(p);
-    if (h->d.err_host) give_flag(h->d.err_host);
+    if (h->d.err_host) cb_give_flag(h->d.err_host);
     if (h->d.st_chcol) cudaFree(h->d.st_chcol);
     if (h->d.pre_jump) cudaFree(h->d.pre_jump);
     cb_resident_free(h->d);

@@ -114,6 +114,10 @@ cudaError_t cb_sg_net_forward(struct casim_surrogate_s* net, const float* x, int
 cudaError_t cb_sg_net_error(struct casim_surrogate_s* net);
 const void* cb_sg_net_output(struct casim_surrogate_s* net);  // changes when its buffers are reallocated
 
+// Error words that kernels with bounded waits set, in mapped host memory (capi.cu); null: none to be had
+int* cb_take_flag();
+void cb_give_flag(int* f);
+
 // resident path (resident.cu)
 bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why);
 cudaError_t cb_resident_step(cb_dev& d, long long n, cudaStream_t st, long long* launches);

@@ -818,36 +818,38 @@ cudaError_t launch_step(cb_dev& d, cudaStream_t st, bool first, bool last, cudaE
 
 // ---- surrogate-driven gating (no RD): the mouth Ca comes from the surrogate network
 
-// features of every site (one thread per site): per RyR slot its open flag and
+// features of every site (one thread per feature): per RyR slot its open flag and
 // grid position scaled to [-1, 1] by the cleft half-widths, then the jSR Ca of
 // the first ion / 1000 uM, then each dyad buffer total relative to its config value
 __global__ void k_sg_features(int S, int n_buf, int max_ch, int ld, const cb_site* __restrict__ sites, const int* __restrict__ ch_node,
                               const int* __restrict__ ch_state, const cb_site_scalars* __restrict__ sc, float* __restrict__ X) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const cb_site st = sites[s];
-    float* row = X + (size_t)s * ld;
-    for (int k = 0; k < ld; ++k) row[k] = 0.0f;
-    const float hx = 0.5f * (st.nx - 1), hy = 0.5f * (st.ny - 1);
-    for (int c = 0; c < st.n_ch && c < max_ch; ++c) {
-        const int node = ch_node[st.ch_off + c];
-        const int gx = node % st.px, gy = (node / st.px) % st.ny;
-        row[3 * c] = (float)ch_state[st.ch_off + c];
-        row[3 * c + 1] = (gx - hx) / hx;
-        row[3 * c + 2] = (gy - hy) / hy;
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= (long long)S * ld) return;
+    const int s = (int)(i / ld), k = (int)(i - (long long)s * ld), c = k / 3, what = k - 3 * c;
+    float v = 0.0f;
+    if (k < 3 * max_ch) {
+        const cb_site st = sites[s];
+        if (c < st.n_ch) {
+            const int node = ch_node[st.ch_off + c];
+            const float hx = 0.5f * (st.nx - 1), hy = 0.5f * (st.ny - 1);
+            v = what == 0 ? (float)ch_state[st.ch_off + c] : what == 1 ? (node % st.px - hx) / hx : ((node / st.px) % st.ny - hy) / hy;
+        }
+    } else if (k == 3 * max_ch) {
+        v = (float)(sc[s].jsr_new[0] / 1000.0);
+    } else if (k <= 3 * max_ch + n_buf) {
+        v = 1.0f;
     }
-    row[3 * max_ch] = (float)(sc[s].jsr_new[0] / 1000.0);
-    for (int b = 0; b < n_buf; ++b) row[3 * max_ch + 1 + b] = 1.0f;
+    X[i] = v;
 }
 
-// mouth Ca of every RyR from the network output: ca_ref * 10^y
+// mouth Ca of every RyR from the network output: ca_ref * 10^y (a thread per site and slot)
 __global__ void k_sg_mouth(int S, int NS, int ca_idx, double ca_ref, int ld, const cb_site* __restrict__ sites,
-                           const float* __restrict__ Y, double* __restrict__ mouth) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+                           const float* __restrict__ Y, double* __restrict__ mouth, int slots) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int s = (int)(i / slots), c = (int)(i - (long long)s * slots);
     if (s >= S) return;
     const cb_site st = sites[s];
-    for (int c = 0; c < st.n_ch && c < ld; ++c)
-        mouth[(size_t)(st.ch_off + c) * NS + ca_idx] = ca_ref * exp10((double)Y[(size_t)s * ld + c]);
+    if (c < st.n_ch) mouth[(size_t)(st.ch_off + c) * NS + ca_idx] = ca_ref * exp10((double)Y[(size_t)s * ld + c]);
 }
 
 // n time steps of one site without the RD step: cytosol pool and jSR ODEs and
@@ -979,12 +981,13 @@ cudaError_t cb_gather_mouth(const cb_dev& d, int species, double* out, cudaStrea
 }
 
 cudaError_t cb_sg_features(cb_dev& d, int max_ch, int ld, float* X, cudaStream_t st) {
-    k_sg_features<<<(d.S + 127) / 128, 128, 0, st>>>(d.S, d.m.n_buf, max_ch, ld, d.sites, d.ch_node, d.ch_state, d.sc, X);
+    k_sg_features<<<(unsigned)(((long long)d.S * ld + 255) / 256), 256, 0, st>>>(d.S, d.m.n_buf, max_ch, ld, d.sites, d.ch_node, d.ch_state, d.sc, X);
     return cudaGetLastError();
 }
 
 cudaError_t cb_sg_mouth(cb_dev& d, const float* Y, int ld, double ca_ref, cudaStream_t st) {
-    k_sg_mouth<<<(d.S + 127) / 128, 128, 0, st>>>(d.S, d.NS, d.m.ca_idx, ca_ref, ld, d.sites, Y, d.mouth);
+    const int slots = std::max(1, std::min(d.max_ch, ld));
+    k_sg_mouth<<<(unsigned)(((long long)d.S * slots + 255) / 256), 256, 0, st>>>(d.S, d.NS, d.m.ca_idx, ca_ref, ld, d.sites, Y, d.mouth, slots);
     return cudaGetLastError();
 }
 

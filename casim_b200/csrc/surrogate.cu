@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/casim_b200.h"
+#include "engine.h"
 
 namespace cbsg {
 
@@ -225,6 +226,141 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(const __grid_constant__ gem
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
 }
 
+// ---- the whole network in one launch (inference)
+// A CTA takes 128 rows through all layers: the activations stay in shared memory (BF16, the
+// canonical layout of the products' A operand, rounded where the layer-by-layer kernels round),
+// the weights stream from L2 in K slices of 64, three stages ahead of the tensor core and across
+// the layer boundary, so that the next layer's first slices load during an epilogue. The products
+// run over the same K order into one TMEM accumulator, so the outputs equal the layer-by-layer
+// ones. 16384 rows of the 63 -> 4 x 256 -> 20 network through the public call: 194 us as a cast, five
+// products, a copy of the used columns and an error read-back, 71 us this way; what remains is the
+// GELU epilogues (erf on the FP32 pipe, about 4.5 us a layer) and the call's synchronisation.
+constexpr int MLP_LAYERS = 16, MLP_THREADS = 256, MLP_STAGES = 3;
+constexpr int MLP_B_STAGE = 256 * BK * 2;  // 32 KiB
+constexpr int MLP_SMEM = 4 * A_STAGE + MLP_STAGES * MLP_B_STAGE;
+struct mlp_args {
+    const float* x;  // [rows][n_in]
+    float* y;        // [rows][ldy], the first ncols columns of the output layer
+    int n_in, in_pad, ldy, ncols, L;
+    int dout[MLP_LAYERS];
+    const bf16* W[MLP_LAYERS];   // [dout][din]
+    const float* b[MLP_LAYERS];
+    int* err;
+};
+
+__global__ void __launch_bounds__(MLP_THREADS, 1) k_mlp(const __grid_constant__ mlp_args g) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bars[MLP_STAGES];
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * BM;
+    const uint32_t sa = smem_u32(smem), sb = sa + 4 * A_STAGE;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(256) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < MLP_STAGES; ++i) mbar_init(&bars[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // weight slice (layer ll, K slice kk) into its stage; the slices of all layers are numbered through
+    int ll = 0, kk = 0, nq = 0, dinl = g.in_pad;
+    auto load_next = [&]() {
+        if (ll < g.L) {
+            const bf16* w = g.W[ll] + kk * BK;
+            const uint32_t d = sb + (nq % MLP_STAGES) * MLP_B_STAGE;
+            for (int p = tid; p < g.dout[ll] * (BK / 8); p += MLP_THREADS) {
+                const int r = p >> 3, c = p & 7;
+                cp_async16(d + (r >> 3) * SBO + c * LBO + (r & 7) * 16, w + (size_t)r * dinl + c * 8);
+            }
+            ++nq;
+            if (++kk == dinl / BK) {
+                kk = 0;
+                dinl = g.dout[ll++];
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_next();
+    load_next();
+    // the input as BF16, zero beyond n_in
+    for (int p = tid; p < BM * g.in_pad / 8; p += MLP_THREADS) {
+        const int n8 = g.in_pad / 8, r = p / n8, c8 = p - r * n8;
+        __align__(16) bf16 h[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = c8 * 8 + j;
+            h[j] = __float2bfloat16_rn(c < g.n_in ? g.x[(size_t)(m0 + r) * g.n_in + c] : 0.0f);
+        }
+        *(uint4*)(smem + (c8 >> 3) * A_STAGE + (r >> 3) * SBO + (c8 & 7) * LBO + (r & 7) * 16) = *(const uint4*)h;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    bool ok = true;
+    int q = 0, din = g.in_pad;
+    for (int l = 0; l < g.L; ++l) {
+        const uint32_t idesc = idesc_bf16(g.dout[l]);
+        for (int k = 0; k < din / BK; ++k, ++q) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");  // slice q is here (q + 1 may be in flight)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+            const int st = q % MLP_STAGES;
+            if (tid == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a = sa + k * A_STAGE, b = sb + st * MLP_B_STAGE;
+#pragma unroll
+                for (int j = 0; j < BK / 16; ++j)
+                    mma_bf16(tmem, sdesc(a + j * 2 * LBO), sdesc(b + j * 2 * LBO), idesc, (k > 0 || j > 0) ? 1u : 0u);
+                mma_commit(&bars[st]);
+            }
+            // slice q + 2 goes where slice q - 1 was
+            if (q >= 1) ok = mbar_wait(&bars[(q - 1) % MLP_STAGES], (uint32_t)(((q - 1) / MLP_STAGES) & 1)) && ok;
+            load_next();
+        }
+        ok = mbar_wait(&bars[(q - 1) % MLP_STAGES], (uint32_t)(((q - 1) / MLP_STAGES) & 1)) && ok;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // epilogue: two warps per lane quarter, half of the columns each
+        const int row = (warp & 3) * 32 + lane, half = g.dout[l] / 2;
+        const int cb = (warp >> 2) * half;
+        const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const bool last = l + 1 == g.L;
+        for (int c0 = cb; c0 < cb + half; c0 += 16) {
+            uint32_t r[16];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(taddr + c0));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (last) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (ok && c0 + j < g.ncols) g.y[(size_t)(m0 + row) * g.ldy + c0 + j] = __uint_as_float(r[j]) + g.b[l][c0 + j];
+            } else {
+#pragma unroll
+                for (int o = 0; o < 16; o += 8) {
+                    __align__(16) bf16 h[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16_rn(gelu(__uint_as_float(r[o + j]) + g.b[l][c0 + o + j]));
+                    const int c = c0 + o;
+                    *(uint4*)(smem + (c >> 6) * A_STAGE + (row >> 3) * SBO + ((c & 63) >> 3) * LBO + (row & 7) * 16) = *(const uint4*)h;
+                }
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        din = g.dout[l];
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!ok && g.err) atomicExch(g.err, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+}
+
 // X FP32 [B][n_in] -> BF16 [B][ld] (zero padded) and its transpose [ld][B]
 __global__ void k_cast_in(const float* __restrict__ x, int B, int n_in, int ld, bf16* __restrict__ xb, bf16* __restrict__ xt) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -376,12 +512,14 @@ struct casim_surrogate_s {
     float* partial = nullptr;
     std::vector<float*> dWp;                             // [splits][dout][din]: K slices of the weight gradients
     float* loss = nullptr;
-    int* err = nullptr;
+    int* err_host = nullptr;  // set to 1 by a kernel whose bounded wait ran out (mapped host memory)
+    int* err = nullptr;       // its device address
     long long step = 0;
     long long launches = 0;
     cudaStream_t stream = 0;
     std::string last_error;
     size_t smem_max = 0;
+    bool mlp_ready = false;  // k_mlp's shared memory is set
 };
 
 namespace {
@@ -435,7 +573,8 @@ unsigned long long splitmix(unsigned long long& s) {
 
 // K slices of a weight gradient [N][K] over a batch of B rows: with one CTA per tile and all of B
 // in sequence, the four tiles of a 256 x 256 layer walked 64 slices each, two thirds of a training
-// step of 4096 rows. About one tile-slice per SM, at least 128 rows each (1060 us per step -> 240).
+// step of 4096 rows. About one tile-slice per SM, at least 128 rows each (four steps and the
+// parameters read back: 4.28 ms before, 1.78 ms with this, the bias sums and the Adam launch).
 int slice_of(int N, int K, int B) {
     const int tiles = N / BM * (K / tile_n(K));
     const int want = (int)(((long long)B * tiles / 148 + BK - 1) / BK * BK);
@@ -481,6 +620,37 @@ cudaError_t ensure_capacity(casim_sg h, int B) {
     if ((e = dalloc(&h->partial, (size_t)B * h->out_pad / 256 + 1)) != cudaSuccess) return e;
     h->cap = B;
     return cudaSuccess;
+}
+
+// inference: the whole network in one launch; y [B][ldy], ncols columns of it written
+bool one_launch(const casim_surrogate_s* h) {
+    bool ok = h->L <= MLP_LAYERS;
+    for (int l = 0; l < h->L; ++l) ok = ok && h->dout[l] % 32 == 0;
+    return ok;
+}
+cudaError_t infer(casim_sg h, const float* x, int B, float* y, int ldy, int ncols) {
+    mlp_args g{};
+    g.x = x;
+    g.y = y;
+    g.n_in = h->n_in;
+    g.in_pad = h->in_pad;
+    g.ldy = ldy;
+    g.ncols = ncols;
+    g.L = h->L;
+    for (int l = 0; l < h->L; ++l) {
+        g.dout[l] = h->dout[l];
+        g.W[l] = h->Wb[l];
+        g.b[l] = h->b[l];
+    }
+    g.err = h->err;
+    if (!h->mlp_ready) {
+        const cudaError_t e = cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM);
+        if (e != cudaSuccess) return e;
+        h->mlp_ready = true;
+    }
+    k_mlp<<<B / BM, MLP_THREADS, MLP_SMEM, h->stream>>>(g);
+    h->launches++;
+    return cudaGetLastError();
 }
 
 // forward through all layers; training keeps Z and H^T for the backward pass
@@ -595,11 +765,9 @@ cudaError_t backward(casim_sg h, const float* t, int B) {
 }
 
 cudaError_t check_err(casim_sg h) {
-    int v = 0;
-    cudaError_t e = cudaMemcpyAsync(&v, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return e;
-    return v ? cudaErrorLaunchTimeout : cudaSuccess;
+    return *(volatile int*)h->err_host ? cudaErrorLaunchTimeout : cudaSuccess;
 }
 
 }  // namespace
@@ -616,7 +784,7 @@ cudaError_t cb_sg_net_forward(casim_sg h, const float* x, int batch, cudaStream_
     if (!h || batch > h->cap) return cudaErrorInvalidValue;
     const cudaStream_t keep = h->stream;
     h->stream = st;
-    const cudaError_t e = forward(h, x, batch, false);
+    const cudaError_t e = one_launch(h) ? infer(h, x, batch, h->Y, h->out_pad, h->out_pad) : forward(h, x, batch, false);
     h->stream = keep;
     *y = h->Y;
     *ld = h->out_pad;
@@ -672,9 +840,9 @@ casim_status casim_b200_sg_create(int n_in, int n_out, int width, int depth, uin
         e = dalloc(&h->Wb[l], (size_t)h->din[l] * h->dout[l]);
         if (e == cudaSuccess) e = dalloc(&h->WTb[l], (size_t)h->din[l] * h->dout[l]);
     }
-    if (e == cudaSuccess) e = dalloc(&h->err, 1);
+    if (e == cudaSuccess && !(h->err_host = cb_take_flag())) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&h->err, h->err_host, 0);
     if (e == cudaSuccess) e = dalloc(&h->loss, 1);
-    if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
     // He-uniform initialisation from a splitmix64 stream; padded rows and columns are zero
     unsigned long long st = (unsigned long long)seed;
     for (int l = 0; l < h->L && e == cudaSuccess; ++l) {
@@ -722,7 +890,7 @@ casim_status casim_b200_sg_destroy(casim_sg h) {
     fr(h->partial);
     for (float* p : h->dWp) fr(p);
     fr(h->loss);
-    fr(h->err);
+    if (h->err_host) cb_give_flag(h->err_host);
     delete h;
     return CASIM_OK;
 }
@@ -772,7 +940,13 @@ casim_status casim_b200_sg_set_params(casim_sg h, const float* host) { return pa
 
 casim_status casim_b200_sg_forward(casim_sg h, const float* x_dev, int batch, float* y_dev) {
     if (!h || !x_dev || !y_dev || batch <= 0 || batch % BM) return CASIM_EINVAL;
-    cudaError_t e = ensure_capacity(h, batch);
+    cudaError_t e = cudaSuccess;
+    if (one_launch(h)) {
+        e = infer(h, x_dev, batch, y_dev, h->n_out, h->n_out);
+        if (e == cudaSuccess) e = check_err(h);
+        return e == cudaSuccess ? CASIM_OK : fail(h, e == cudaErrorLaunchTimeout ? CASIM_ETIMEOUT : CASIM_ECUDA, cudaGetErrorString(e));
+    }
+    e = ensure_capacity(h, batch);
     if (e == cudaSuccess) e = forward(h, x_dev, batch, false);
     if (e == cudaSuccess)
         e = cudaMemcpy2DAsync(y_dev, (size_t)h->n_out * 4, h->Y, (size_t)h->out_pad * 4, (size_t)h->n_out * 4, batch,
@@ -837,10 +1011,9 @@ casim_status casim_b200_sg_last_error(casim_sg h, char* buf, size_t n) {
 casim_status casim_b200_sg_gemm(const void* a_dev, const void* b_dev, int M, int N, int K, float* c_dev) {
     if (!a_dev || !b_dev || !c_dev) return CASIM_EINVAL;
     casim_surrogate_s tmp;
-    int* err = nullptr;
-    if (cudaMalloc(&err, sizeof(int)) != cudaSuccess) return CASIM_ENOMEM;
-    cudaMemset(err, 0, sizeof(int));
-    tmp.err = err;
+    tmp.err_host = cb_take_flag();
+    if (!tmp.err_host) return CASIM_ENOMEM;
+    cudaError_t e = cudaHostGetDevicePointer((void**)&tmp.err, tmp.err_host, 0);
     gemm_args g{};
     g.A = (const bf16*)a_dev;
     g.B = (const bf16*)b_dev;
@@ -849,10 +1022,10 @@ casim_status casim_b200_sg_gemm(const void* a_dev, const void* b_dev, int M, int
     g.K = K;
     g.mode = EPI_PLAIN;
     g.C = c_dev;
-    g.err = err;
-    cudaError_t e = gemm(&tmp, g);
+    g.err = tmp.err;
+    if (e == cudaSuccess) e = gemm(&tmp, g);
     if (e == cudaSuccess) e = check_err(&tmp);
-    cudaFree(err);
+    cb_give_flag(tmp.err_host);
     if (e == cudaErrorInvalidValue) return CASIM_EINVAL;
     return e == cudaSuccess ? CASIM_OK : e == cudaErrorLaunchTimeout ? CASIM_ETIMEOUT : CASIM_ECUDA;
 }
