@@ -364,8 +364,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         }
         if (tid == 32) {
             // Update rim tasks: 32 consecutive nodes of one line, dealt chunk-major so that
-            // the long y-edge lines of the first and last rank spread over the warps (one-block
-            // sites: whole lines, one task each)
+            // the long y-edge lines of the first and last rank spread over the warps
             const int zm = NZ == 1 ? 1 : nz - 1;
             const int nrw = max(min(hi, ny - 1) - max(lo, 1), 0);
             int nt = 0;
@@ -381,7 +380,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                         any = true;
                     }
                 }
-                if (!any || C == 1) break;
+                if (!any) break;
             }
             s_nlt = nt;
         }
@@ -453,6 +452,32 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         const fastdiv fd_nxi = make_fastdiv(max(nxi, 1)), fd_ncol = make_fastdiv(max(ncol, 1)), fd_ni = make_fastdiv(max(ni, 1));
         cluster_barrier<C>();
 
+        // The previous Update's sums: of the ranks' partials in rank order, the same on every rank;
+        // one-block sites sum the warps' partials here, four interleaved sums in a fixed order,
+        // which saves them a block barrier and a serial sum at the end of every step.
+        auto warps_sum = [&](int k) {
+            double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+            for (int w = 0; w < W; w += 4) {
+                s0 += redw[w * FDn + k];
+                if (w + 1 < W) s1 += redw[(w + 1) * FDn + k];
+                if (w + 2 < W) s2 += redw[(w + 2) * FDn + k];
+                if (w + 3 < W) s3 += redw[(w + 3) * FDn + k];
+            }
+            return (s0 + s1) + (s2 + s3);
+        };
+        auto efflux_of = [&](int par, int f) {
+            if constexpr (C == 1) return warps_sum(f);
+            double e = 0;
+            for (int r = 0; r < C; ++r) e += rede[(par * C + r) * F + f];
+            return e;
+        };
+        auto total_of = [&](int par, int j) {
+            if constexpr (C == 1) return warps_sum(F + j);
+            double t = 0;
+            for (int r = 0; r < C; ++r) t += redt[(par * C + r) * NI + j];
+            return t;
+        };
+
         // ---------------------------------------------------------- steps
         for (long long it = 0; it < a.nsteps; ++it) {
             const int par = (int)(it & 1), prv = par ^ 1;
@@ -501,19 +526,10 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                 }
                 __syncwarp();
                 if (lane == 0) s_D = D;
-            } else if (warp == 1) {
-                // ---- pools: reductions of the previous Update (rank order on every rank)
+                // ---- jSR: coupling to the previous Update's currents, then its ODE
+                // (CaSim/SRPool.cpp:55-89) with the site's own beta
                 if (it > 0) {
-                    for (int f = lane; f < F; f += 32) {
-                        double e = 0;
-                        for (int r = 0; r < C; ++r) e += rede[(prv * C + r) * F + f];
-                        q.efflux[f] = e;
-                    }
-                    for (int j = lane; j < NI; j += 32) {
-                        double t = 0;
-                        for (int r = 0; r < C; ++r) t += redt[(prv * C + r) * NI + j];
-                        q.total[j] = t;
-                    }
+                    if (lane < NI) q.total[lane] = total_of(prv, lane);
                     __syncwarp();
                     if (lane == 0 && !m.jsr_const)
                         for (int i = 0; i < NI; ++i) {
@@ -521,6 +537,22 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                             q.nsr[i] = m.nsr[i];
                             q.jsr[i] = q.jsr_new[i];
                         }
+                }
+                if (lane == 0 && !m.jsr_const) {
+                    double beta = 1;
+                    for (int j = 0; j < NI; ++j)
+                        beta += m.nCQ[j] * m.K_CQ[j] * m.CQ / ((m.K_CQ[j] + q.jsr[j]) * (m.K_CQ[j] + q.jsr[j]));
+                    for (int i = 0; i < NI; ++i) {
+                        const double Iref = 1 / m.tau_refill[i] * (q.nsr[i] - q.jsr[i]);
+                        q.jsr_new[i] = q.jsr[i] + dt / beta * (Iref - q.IjSR[i] / m.V_jsr);
+                    }
+                    if (m.ca_idx >= 0) q.release += q.IjSR[m.ca_idx] * dt;
+                }
+                __syncwarp();
+            } else if (warp == 1) {
+                // ---- cytosol pool: the previous Update's efflux, then its ODE
+                if (it > 0) {
+                    for (int f = lane; f < F; f += 32) q.efflux[f] = efflux_of(prv, f);
                     __syncwarp();
                 }
                 if (lane == 0) {
@@ -558,17 +590,6 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                         }
                         for (int b = 0; b < m.c_n_buf; ++b) q.c_free[b] = m.c_Ctot[b];
                         for (int p = 0; p < m.c_n_pairs; ++p) q.c_free[m.c_pair_buf[p]] -= q.c_pairs[p];
-                    }
-                    // jSR ODE (CaSim/SRPool.cpp:70-89) with the site's own beta
-                    if (!m.jsr_const) {
-                        double beta = 1;
-                        for (int j = 0; j < NI; ++j)
-                            beta += m.nCQ[j] * m.K_CQ[j] * m.CQ / ((m.K_CQ[j] + q.jsr[j]) * (m.K_CQ[j] + q.jsr[j]));
-                        for (int i = 0; i < NI; ++i) {
-                            const double Iref = 1 / m.tau_refill[i] * (q.nsr[i] - q.jsr[i]);
-                            q.jsr_new[i] = q.jsr[i] + dt / beta * (Iref - q.IjSR[i] / m.V_jsr);
-                        }
-                        if (m.ca_idx >= 0) q.release += q.IjSR[m.ca_idx] * dt;
                     }
                 }
                 if (rd3d) {
@@ -821,9 +842,12 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
             //                    over x in [1, nx-2] where this rank holds them
             //   l - 4*nz < 4*zmax  efflux terms (CaSim/DyadRD2DCPU.cpp:305-350) in the same edge order:
             //                    e 0/1 over y in [ylo, yhi); e 2/3 over x in [0, nx-1]
-            double epart[CSM];
+            double epart[CSM], ef[CSM];  // pool: D * grad_mult
 #pragma unroll
-            for (int f = 0; f < CSM; ++f) epart[f] = 0;
+            for (int f = 0; f < CSM; ++f) {
+                epart[f] = 0;
+                ef[f] = f < F ? (f < NI ? m.D_ion[f] : m.D_pair[f - NI]) * m.grad_mult : 0;
+            }
             {
                 R* t0 = peer<C>(terms + (size_t)par * a.max_terms * FD, r0);
                 // one-block sites: the last warps hold the channels (and their rate laws), so
@@ -849,7 +873,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                             dxs = 1;
                             ri0 = 2 * ny + (e == 2 ? 0 : nx - 2);
                         }
-                        for (int i = i0 + lane; i < (C == 1 ? len : min(len, i0 + 32)); i += 32) {
+                        for (int i = i0 + lane; i < min(len, i0 + 32); i += 32) {
                             const int x = x0 + dxs * i, y = y0 + (1 - dxs) * i;
                             const int n = x + nx * ((y - slo) + nr * z);
 #pragma unroll
@@ -876,7 +900,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                             sf = m.sy;
                             gt0 = (2 * (ny - 2) + (e - 2) * nx) * zmax + z;
                         }
-                        for (int i = i0 + lane; i < (C == 1 ? len : min(len, i0 + 32)); i += 32) {
+                        for (int i = i0 + lane; i < min(len, i0 + 32); i += 32) {
                             // the edge node walks along the line: y for x-edges, x for y-edges
                             const int xe = e < 2 ? x0 : i, ye = e < 2 ? y0 + i : y0;
                             const int ri = e < 2 ? (e ? ny : 0) + ye
@@ -897,7 +921,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                                     const double u2 = rc >= 0 ? (double)rim_value(f, rc + ye + 2 * dys) : (double)fb[f * cap + n2];
                                     const double gr = 2 * u1 - 1.5 * u0 - 0.5 * u2;
                                     if (!rd3d) {
-                                        epart[f] += D * m.grad_mult * sf * gr;
+                                        epart[f] += ef[f] * sf * gr;
                                     } else {
                                         const double v = D * sf * gr * m.inv_hc3;
                                         epart[f] += v;
@@ -972,34 +996,22 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                     for (int j = 0; j < NI; ++j) redw[warp * FDn + F + j] = wv[CSM + j];
                 }
             }
-            __syncthreads();
-            // rank partials (fixed warp order) into every rank's slot
-            if (warp == 0) {
-                double v = 0;
-                if (lane < FDn) {
-                    // four interleaved sums over the warps (a fixed order: every run and every
-                    // rank forms the same total)
-                    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-                    for (int w = 0; w < W; w += 4) {
-                        s0 += redw[w * FDn + lane];
-                        if (w + 1 < W) s1 += redw[(w + 1) * FDn + lane];
-                        if (w + 2 < W) s2 += redw[(w + 2) * FDn + lane];
-                        if (w + 3 < W) s3 += redw[(w + 3) * FDn + lane];
-                    }
-                    v = (s0 + s1) + (s2 + s3);
-                }
-                // FDn (at most 20) values x C ranks: one store per lane
-                for (int b0 = 0; b0 < FDn * C; b0 += 32) {
-                    const int idx = b0 + lane;
-                    const int k = idx / C, r = idx - k * C;
-                    const double vk = __shfl_sync(0xffffffffu, v, k < FDn ? k : 0);
-                    if (idx < FDn * C) {
-                        if (k < F) peer<C>(rede, r)[(par * C + rank) * F + k] = vk;
-                        else peer<C>(redt, r)[(par * C + rank) * NI + (k - F)] = vk;
-                    }
-                }
-            }
             if constexpr (C > 1) {
+                __syncthreads();
+                // rank partials (fixed warp order) into every rank's slot
+                if (warp == 0) {
+                    const double v = lane < FDn ? warps_sum(lane) : 0;
+                    // FDn (at most 20) values x C ranks: one store per lane
+                    for (int b0 = 0; b0 < FDn * C; b0 += 32) {
+                        const int idx = b0 + lane;
+                        const int k = idx / C, r = idx - k * C;
+                        const double vk = __shfl_sync(0xffffffffu, v, k < FDn ? k : 0);
+                        if (idx < FDn * C) {
+                            if (k < F) peer<C>(rede, r)[(par * C + rank) * F + k] = vk;
+                            else peer<C>(redt, r)[(par * C + rank) * NI + (k - F)] = vk;
+                        }
+                    }
+                }
                 // halo rows into the neighbours' write buffers, a warp per (species, layer) row
                 for (int side = 0; side < 2; ++side) {
                     const int nb = side == 0 ? rank - 1 : rank + 1;
@@ -1051,16 +1063,8 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
         // ---------------------------------------------------------- store
         if (warp == 0 && a.nsteps > 0) {
             const int pl = (int)((a.nsteps - 1) & 1);
-            for (int f = lane; f < F; f += 32) {
-                double e = 0;
-                for (int r = 0; r < C; ++r) e += rede[(pl * C + r) * F + f];
-                q.efflux[f] = e;
-            }
-            for (int j = lane; j < NI; j += 32) {
-                double t = 0;
-                for (int r = 0; r < C; ++r) t += redt[(pl * C + r) * NI + j];
-                q.total[j] = t;
-            }
+            for (int f = lane; f < F; f += 32) q.efflux[f] = efflux_of(pl, f);
+            if (lane < NI) q.total[lane] = total_of(pl, lane);
             __syncwarp();
             if (lane == 0) {
                 if (!m.jsr_const)
