@@ -70,6 +70,8 @@ struct cb_model {
     double grad_mult;  // 3/(4 pi R^3)
     double sx, sy;     // edge face factors of the efflux
     double V_elem;     // DyadSeries::GetElementVolume
+    double inv_tau[CB_MAX_IONS], inv_V_jsr;  // 1 / tau_refill, 1 / V_jsr
+    double c_rest[CB_MAX_IONS];              // by SERCA index: uptake share at rest, bg^2 / (bg^2 + Kup^2)
     double inv_dx2, inv_dy2, inv_dz2, inv_hc2, inv_hc3;
 };
 

@@ -450,6 +450,12 @@ cb_config cb_parse_config(const std::string& json_text, const std::string& base_
         m.sy = m.dx * m.dz / m.dy;
         m.V_elem = 0.5 * m.dx * m.dy * m.dz;  // CaSim/DyadRDCPU.cpp:195-197
     }
+    for (int i = 0; i < CB_MAX_IONS; ++i) {
+        m.inv_tau[i] = 1 / m.tau_refill[i];
+        const double b2 = m.c_bg[i] * m.c_bg[i];
+        m.c_rest[i] = b2 / (b2 + m.c_Kup[i] * m.c_Kup[i]);
+    }
+    m.inv_V_jsr = 1 / m.V_jsr;
     m.inv_dx2 = 1.0 / (m.dx * m.dx);
     m.inv_dy2 = 1.0 / (m.dy * m.dy);
     m.inv_dz2 = 1.0 / (m.dz * m.dz);

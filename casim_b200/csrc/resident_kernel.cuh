@@ -35,6 +35,7 @@
 #include "engine.h"
 #include "mrg32k3a.cuh"
 #include "physics.cuh"
+#include "pools.cuh"
 
 namespace cbres {
 
@@ -193,6 +194,7 @@ template <typename R, int NI, int NPM, int NZ, int C>
 __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_resident(const __grid_constant__ rs_args a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_site;
+    __shared__ R s_rim[NI + NPM];  // pool cytosol: this step's Dirichlet values
     // RNG of warp 0, kept in shared memory so it holds no registers during the stencils:
     // lane l's stream at draw s_we + l*LANE_DRAWS; s_D draws consumed
     __shared__ unsigned int s_rng[32 * 6];
@@ -538,16 +540,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                             q.jsr[i] = q.jsr_new[i];
                         }
                 }
-                if (lane == 0 && !m.jsr_const) {
-                    double beta = 1;
-                    for (int j = 0; j < NI; ++j)
-                        beta += m.nCQ[j] * m.K_CQ[j] * m.CQ / ((m.K_CQ[j] + q.jsr[j]) * (m.K_CQ[j] + q.jsr[j]));
-                    for (int i = 0; i < NI; ++i) {
-                        const double Iref = 1 / m.tau_refill[i] * (q.nsr[i] - q.jsr[i]);
-                        q.jsr_new[i] = q.jsr[i] + dt / beta * (Iref - q.IjSR[i] / m.V_jsr);
-                    }
-                    if (m.ca_idx >= 0) q.release += q.IjSR[m.ca_idx] * dt;
-                }
+                if (lane == 0) cb_jsr_step<NI>(m, q, dt);
                 __syncwarp();
             } else if (warp == 1) {
                 // ---- cytosol pool: the previous Update's efflux, then its ODE
@@ -557,39 +550,9 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                 }
                 if (lane == 0) {
                     if (!rd3d) {
-                        // cytosol pool ODE (CaSim/CytosolPool.cpp:217-288)
-                        double evo_i[CB_MAX_IONS], evo_p[CB_MAX_CPAIRS];
-                        int ipd = 0, is = 0;
-                        for (int j = 0; j < NI; ++j) {
-                            double react = 0;
-                            for (int p = 0; p < m.c_n_pairs; ++p) {
-                                if (m.c_pair_ion[p] != j) continue;
-                                const double R1 = m.c_koff[p] * q.c_pairs[p] - m.c_kon[p] * q.c_ions[j] * q.c_free[m.c_pair_buf[p]];
-                                evo_p[p] = -R1;
-                                react += R1;
-                                if (m.c_in_dyad[p]) evo_p[p] += q.efflux[NI + ipd++];
-                            }
-                            evo_i[j] = react + q.efflux[j];
-                            if (m.c_serca[j]) {
-                                const double i2 = q.c_ions[j] * q.c_ions[j];
-                                const double K2 = m.c_Kup[is] * m.c_Kup[is];
-                                const double b2 = m.c_bg[is] * m.c_bg[is];
-                                evo_i[j] -= m.c_Jmax[is] * (i2 / (i2 + K2) - b2 / (b2 + K2));
-                                ++is;
-                            }
-                        }
-                        for (int j = 0; j < NI; ++j) {
-                            evo_i[j] -= m.c_onetau_ion[j] * (q.c_ions[j] - m.c_bg[j]);
-                            q.c_ions[j] += evo_i[j] * dt;
-                        }
-                        ipd = 0;
-                        for (int p = 0; p < m.c_n_pairs; ++p) {
-                            evo_p[p] -= m.c_onetau_pair[p] * (q.c_pairs[p] - m.c_init[p]);
-                            q.c_pairs[p] += evo_p[p] * dt;
-                            if (m.c_in_dyad[p]) q.c_bnd[ipd++] = q.c_pairs[p];
-                        }
-                        for (int b = 0; b < m.c_n_buf; ++b) q.c_free[b] = m.c_Ctot[b];
-                        for (int p = 0; p < m.c_n_pairs; ++p) q.c_free[m.c_pair_buf[p]] -= q.c_pairs[p];
+                        cb_pool_step<NI>(m, q, dt);
+                        for (int j = 0; j < NI; ++j) s_rim[j] = (R)q.c_ions[j];
+                        for (int p = 0; p < NP; ++p) s_rim[NI + p] = (R)q.c_bnd[p];
                     }
                 }
                 if (rd3d) {
@@ -830,7 +793,7 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
             // rim values: the cytosol at the start of this step (pool, or the RD3D
             // layer-0 values gathered in phase A)
             auto rim_value = [&](int f, int ri) -> R {
-                if (!rd3d) return f < NI ? (R)q.c_ions[f] : (R)q.c_bnd[f - NI];
+                if (!rd3d) return s_rim[f];
                 const int u = crim[ri];
                 if (f < NI) return rimc[f * a.max_rim + u];
                 const int cq = m.dyad_c_pair[f - NI];
@@ -848,7 +811,47 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                 epart[f] = 0;
                 ef[f] = f < F ? (f < NI ? m.D_ion[f] : m.D_pair[f - NI]) * m.grad_mult : 0;
             }
-            {
+            if (!rd3d) {
+                // pool cytosol: one value per species on the whole rim, so a thread takes a rim node
+                // with its efflux terms: no tasks, no look-ups (a y-edge line's corner terms are
+                // 2v - 1.5v - 0.5v = 0). The last warps hold the channels of one-block sites.
+                const int WL = C == 1 ? max(1, W - (nch + 31) / 32) : W;
+                const int ns = hi - lo, nt = (lo == 0 ? nx - 2 : 0), nbt = (hi == ny ? nx - 2 : 0);
+                if (warp < WL) {
+                    R rv[CSM];
+#pragma unroll
+                    for (int f = 0; f < CSM; ++f) rv[f] = f < F ? s_rim[f] : (R)0;
+                    for (int i = tid; i < 2 * ns + nt + nbt; i += 32 * WL) {
+                        int x, y, step;
+                        bool term = true;
+                        if (i < 2 * ns) {
+                            const bool far = i >= ns;
+                            x = far ? nx - 1 : 0;
+                            y = lo + i - (far ? ns : 0);
+                            step = far ? -1 : 1;
+                            term = y > 0 && y < ny - 1;
+                        } else {
+                            const bool far = i >= 2 * ns + nt;
+                            x = 1 + i - 2 * ns - (far ? nt : 0);
+                            y = far ? ny - 1 : 0;
+                            step = far ? -nx : nx;
+                        }
+                        const double sf = i < 2 * ns ? m.sx : m.sy;
+                        const int n0 = x + nx * (y - slo);
+                        for (int z = 0; z < nz; ++z) {
+                            const int n = n0 + lstride * z;
+#pragma unroll
+                            for (int f = 0; f < CSM; ++f)
+                                if (f < F) {
+                                    fb[f * cap + n] = rv[f];
+                                    if (term && z < zmax)
+                                        epart[f] += ef[f] * sf * (2 * (double)fb[f * cap + n + step] - 1.5 * (double)rv[f] -
+                                                                  0.5 * (double)fb[f * cap + n + 2 * step]);
+                                }
+                        }
+                    }
+                }
+            } else {
                 R* t0 = peer<C>(terms + (size_t)par * a.max_terms * FD, r0);
                 // one-block sites: the last warps hold the channels (and their rate laws), so
                 // the tasks go to the others
@@ -920,14 +923,10 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                                     const double u1 = rc >= 0 ? (double)rim_value(f, rc + ye + dys) : (double)fb[f * cap + n1];
                                     const double u2 = rc >= 0 ? (double)rim_value(f, rc + ye + 2 * dys) : (double)fb[f * cap + n2];
                                     const double gr = 2 * u1 - 1.5 * u0 - 0.5 * u2;
-                                    if (!rd3d) {
-                                        epart[f] += ef[f] * sf * gr;
-                                    } else {
-                                        const double v = D * sf * gr * m.inv_hc3;
-                                        epart[f] += v;
-                                        const int sl = dslot(m, NI, f);
-                                        if (sl >= 0) t0[tpos[gterm] * FD + sl] = (R)v;
-                                    }
+                                    const double v = D * sf * gr * m.inv_hc3;
+                                    epart[f] += v;
+                                    const int sl = dslot(m, NI, f);
+                                    if (sl >= 0) t0[tpos[gterm] * FD + sl] = (R)v;
                                 }
                             }
                         }

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(64 * SG_WARPS) k_sg_warp(const __grid_constant
     const int nch = st.n_ch;
     if (mine && pool) {
         if (lane == 0 && m.cyto_type == CB_CYTO_POOL)
-            for (long long it = 0; it < n; ++it) cb_pool_step(m, W.q, dt);
+            for (long long it = 0; it < n; ++it) cb_pool_step<NI>(m, W.q, dt);
     } else if (mine) {
         for (int c = lane; c < nch; c += 32) {
             const double* mo = mouth + (size_t)(st.ch_off + c) * NS;
@@ -86,14 +86,10 @@ __global__ void __launch_bounds__(64 * SG_WARPS) k_sg_warp(const __grid_constant
         long long D = 0, we = 0;
         for (long long it = 0; it < n; ++it) {
             if (!m.jsr_const) {
-                double beta = 1;
-#pragma unroll
-                for (int j = 0; j < NI; ++j) beta += m.nCQ[j] * m.K_CQ[j] * m.CQ / ((m.K_CQ[j] + jsr[j]) * (m.K_CQ[j] + jsr[j]));
-                const double db = dt / beta;
+                const double db = cb_jsr_dt_beta<NI>(m, jsr, dt);
 #pragma unroll
                 for (int j = 0; j < NI; ++j) {
-                    const double Iref = 1 / m.tau_refill[j] * (nsr[j] - jsr[j]);
-                    jnew[j] = jsr[j] + db * (Iref - I[j] / m.V_jsr);
+                    jnew[j] = jsr[j] + db * (m.inv_tau[j] * (nsr[j] - jsr[j]) - I[j] * m.inv_V_jsr);
                     if (j == m.ca_idx) release += I[j] * dt;
                 }
             }

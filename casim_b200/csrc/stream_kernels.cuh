@@ -1032,13 +1032,13 @@ __global__ void __launch_bounds__(UP_THREADS, 4)
         gate_warp(st, q, ga.prob, ga.pcm, ga.ch_state, ga.ch_micro, ga.mwc, ga.J, s_ring, s_open);
     } else if (GATE && RD3D && warp == 1) {
         if (lane == 0) {
-            cb_jsr_step(m, q, m.dt);
+            cb_jsr_step<NI>(m, q, m.dt);
 #pragma unroll
             for (int j = 0; j < NI; ++j) s_jsr[j] = q.jsr_new[j];
         }
     } else {
         if (et == 0) {
-            if (GATE && !RD3D) cb_pool_step(m, q, m.dt);
+            if (GATE && !RD3D) cb_pool_step<NI>(m, q, m.dt);
 #pragma unroll
             for (int j = 0; j < NI; ++j) s_rim[j] = (R)q.c_ions[j];
 #pragma unroll
@@ -1156,7 +1156,7 @@ __global__ void __launch_bounds__(UP_THREADS, 4)
         if (POOL) {
             set_rim();
             if (et == 0) {
-                cb_jsr_step(m, q, m.dt);
+                cb_jsr_step<NI>(m, q, m.dt);
             }
         }
         if (!RD3D || !GATE) {
