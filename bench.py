@@ -211,8 +211,10 @@ def dominant_kernel(args, sim, sites, bytes_step, peak):
         for k, v in sim.profile_step().items():
             prof[k] = prof.get(k, 0.0) + v / 5
     kbytes = {"cleft": 2 * w * F * cleft_nodes, "cytosol": 2 * w * CS * sim.S * sim.info.cyto_nodes}
-    names = {"gating": "k_pre_r (RyR gating, pools)", "cytosol": "k_cyto_m (RD3D cytosol)", "cleft": "k_rd_s (cleft stencil)",
-             "update": "k_update_s (Update)"}
+    names = {"gating": "k_prob (first gating probabilities of a call)", "cytosol": "k_cyto_t (RD3D cytosol)",
+             "cleft": "k_rd_t (cleft stencil)", "update": "k_update_s (RyR gating, pools, Update)"}
+    # a call of many steps forms the first probabilities once: their kernel is not a part of the step
+    prof["gating"] = prof.get("gating", 0.0) / max(1, args.chunk)
     dom = max(prof, key=prof.get)
     step_ms = sum(prof.values())
     kernels = {names[k]: {"ms": v, "share": v / step_ms,

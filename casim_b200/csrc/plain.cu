@@ -1,4 +1,6 @@
-// Plain path: one time step = one launch sequence over HBM-resident fields.
+// Plain path: one time step = one launch sequence over HBM-resident fields. Layouts of 1-2 ions, up to
+// 4 pairs and 1 or 3 cleft layers run the specialised kernels of stream_kernels.cuh (cytosol, cleft,
+// gating with pools and Update: two or three launches per step), others the generic ones here:
 //
 //   k_pre     one thread per site: cytosol pool ODE (CaSim/CytosolPool.cpp:217-268),
 //             jSR pool ODE (CaSim/SRPool.cpp:70-89), two-state gating
@@ -9,8 +11,8 @@
 //   k_update  one block per site: mouth gather, Dirichlet edges, efflux,
 //             RyR currents, jSR coupling (CaSim/ParallelHybridSolver.cpp:159-175)
 //
-// This is the straightforward GPU formulation of the reference step and the
-// denominator of the resident path's speed-up; it handles any site size.
+// The generic kernels are the straightforward GPU formulation of the reference step; they
+// handle any site size and layout.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -709,7 +711,8 @@ cudaError_t launch_rd_s(cb_dev& d, cudaStream_t st) {
         auto kern = d.st_nz == 1 ? stream::k_rd_t<R, NI, NP, 1, V, stream::RDT_STAGES> : stream::k_rd_t<R, NI, NP, 3, V, stream::RDT_STAGES>;
         cudaError_t e;
         if (d.st_grid == 0) {
-            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+            // the cap of a kernel is shared by all handles, whose carves differ: always the most
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024)) != cudaSuccess) return e;
             int dev = 0, sms = 0, per = 0;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;

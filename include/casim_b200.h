@@ -247,9 +247,10 @@ casim_status casim_b200_last_step_launches(casim_h h, int64_t* out);
 casim_status casim_b200_set_site_gating(casim_h h, const char* json_text, const char* base_dir, const int32_t* sites, int32_t n);
 /* Profiling (no counterpart in the reference): advance every site by one time step
  * like casim_b200_step(h, 1) and return the device time in ms of each of its kernels,
- * from CUDA events on the handle's stream. Plain path: ms[0..3] = RyR gating and pools,
- * RD3D cytosol (0 without it), cleft stencil, Update; resident path: ms[0] = the one
- * launch. *count receives how many entries were written (at most n). Synchronous; not
+ * from CUDA events on the handle's stream. Plain path: ms[0..3] = RyR gating and pools
+ * (specialised kernels: the probabilities of a call's first gating, the gating itself runs
+ * in the Update), RD3D cytosol (0 without it), cleft stencil, Update; resident path:
+ * ms[0] = the one launch. *count receives how many entries were written (at most n). Synchronous; not
  * while an open-RyR trace is enabled. */
 casim_status casim_b200_profile_step(casim_h h, double* ms, int32_t n, int32_t* count);
 

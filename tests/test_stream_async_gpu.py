@@ -77,6 +77,29 @@ def test_cytosol_chunks_agree(cuda_device, n):
         sim.close()
 
 
+def test_batches_of_different_rows_side_by_side(cuda_device):
+    """Two handles whose tiles need different shared memory, stepped in turn: each equals its own
+    run alone (the kernels' shared-memory cap is common to all handles)."""
+    big, small = configs.config2(n_sites=3, seed=5, side=(110, 120), ryr=(4, 6)), configs.config2(n_sites=3, seed=6, side=(12, 16), ryr=(2, 4))
+    alone = []
+    for p, s in (big, small):
+        sim = cb.ReleaseSiteBatch(p, s, precision="fp32", path="plain")
+        sim.start(s["first_channel"])
+        sim.step(20)
+        alone.append([sim.field(k, 0) for k in range(3)])
+        sim.close()
+    sims = [cb.ReleaseSiteBatch(p, s, precision="fp32", path="plain") for p, s in (big, small)]
+    for sim, (_, s) in zip(sims, (big, small)):
+        sim.start(s["first_channel"])
+    for _ in range(2):
+        for sim in sims:
+            sim.step(10)
+    for sim, want in zip(sims, alone):
+        for k in range(3):
+            assert np.array_equal(sim.field(k, 0), want[k])
+        sim.close()
+
+
 def _compare(p, s, precision, steps):
     sim = cb.ReleaseSiteBatch(json.loads(json.dumps(p)), s, precision=precision, path="plain")
     orc = oracle.OracleSim(p, s)
