@@ -53,6 +53,7 @@ struct casim_b200_sim {
     double last_ms = 0;
     long long last_launches = 0;
     std::vector<void*> allocs;
+    bool streams_by_rounds = false;  // AUTO streams a batch whose state the L2 holds
     std::string resident_why;  // how the resident path splits the batch, or why it was not chosen
     // surrogate-driven gating: feature buffer and one captured window
     float* sg_x = nullptr;
@@ -305,7 +306,8 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
         int thr = 0;
         size_t smem = 0;
         std::string why;
-        bool fits = cb_resident_fits(h->d, &thr, &smem, &why);
+        double rounds = 0;
+        bool fits = cb_resident_fits(h->d, &thr, &smem, &why, &rounds);
         h->resident_why = why;
         if (path == CASIM_PATH_RESIDENT && !fits) {
             std::string msg = "resident path unavailable: " + why;
@@ -314,9 +316,17 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
         }
         h->path = (path == CASIM_PATH_PLAIN || !fits) ? CASIM_PATH_PLAIN : CASIM_PATH_RESIDENT;
         if (path == CASIM_PATH_AUTO && fits) {
-            // large 3D batches stream faster than they run resident (measured on the
-            // 4096-dyad RD3D workload: 146 against 85 site-ms/s; 2D batches of 100 and
-            // 1024 sites: resident 5.5x and 2.7x the streaming path)
+            // Large 3D batches stream faster than they run resident (4096 dyads with the RD3D
+            // cytosol: 0.76 against 2.4 ms a step; 2D batches of 100 and 1024 sites: resident 4.4
+            // and 31 us). Below the L2's size the resident step grows with the rounds in which the
+            // sites take the chip's clusters, about 8.5 us a round with the RD3D cytosol, while the
+            // streaming step starts at its launches' 31 us and grows by 0.25 us a site: streaming
+            // from 4.5 rounds on (us resident / streaming, FP32: sides 40..120, 48 sites, 3.7 rounds
+            // 33.8 / 32.9, 64 sites, 5.1 rounds 42.6 / 34.9; sides 40..60, 3.9 rounds 36.4 / 38.5,
+            // 4.9 rounds 45.8 / 41.9; sides 100..120, 64 sites, 9.1 rounds 79.3 / 39.0; with Mg,
+            // sides 40..60, 256 sites, 17 rounds 167 / 82). With a pool cytosol small sites take
+            // one or two blocks each and stay faster resident (1200 sites of sides 40..60, 11
+            // rounds: 64 / 89).
             const bool rd3d = h->d.m.cyto_type == CB_CYTO_RD3D;
             const size_t w = precision == CASIM_FP64 ? 8 : 4;
             const size_t mc = (size_t)h->d.m.mc;
@@ -324,10 +334,13 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
             int dev = 0, l2 = 0;
             ck(cudaGetDevice(&dev), "cudaGetDevice");
             ck(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev), "cudaDeviceGetAttribute");
-            if ((rd3d || h->d.m.dim == 3) && state > (size_t)l2 && cb_plain_streaming(h->d)) {
+            const bool large = state > (size_t)l2;
+            if ((rd3d || h->d.m.dim == 3) && (large || (rd3d && rounds >= 4.5)) && cb_plain_streaming(h->d)) {
                 h->path = CASIM_PATH_PLAIN;
-                h->resident_why = "streaming: state of " + std::to_string(state >> 20) + " MiB exceeds the " +
-                                  std::to_string(l2 >> 20) + " MiB L2 (resident would be: " + why + ")";
+                h->streams_by_rounds = !large;
+                h->resident_why = "streaming: state of " + std::to_string(state >> 20) + " MiB " + (large ? "exceeds the " : "of the ") +
+                                  std::to_string(l2 >> 20) + " MiB L2" + (large ? "" : ", " + std::to_string((int)rounds) + " rounds of clusters") +
+                                  " (resident would be: " + why + ")";
             }
         }
         ck(cb_plain_reset(h->d, h->stream), "reset");
@@ -564,7 +577,7 @@ casim_status casim_b200_profile_step(casim_h h, double* ms, int32_t n, int32_t* 
 casim_status casim_b200_set_site_gating(casim_h h, const char* json_text, const char* base_dir, const int32_t* sites, int32_t n) {
     GUARD(h)
     if (!json_text || !sites || n < 1) throw std::runtime_error("set_site_gating: bad argument");
-    if (h->path != CASIM_PATH_PLAIN) throw unsupported("per-site gating models run on the plain path (create the handle with it)");
+    if (h->path != CASIM_PATH_PLAIN || h->streams_by_rounds) throw unsupported("per-site gating models run on the plain path (create the handle with it)");
     if (h->d.mwc || h->d.m.ch_model == CB_SINGLE_SITE_MWC) throw unsupported("per-site gating models are two-state models");
     if (!cb_plain_gating_ready(h->d)) throw unsupported("per-site gating models need the specialised streaming kernels");
     for (int k = 0; k < n; ++k) check_site(h, sites[k]);

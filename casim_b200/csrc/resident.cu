@@ -251,7 +251,8 @@ bool classify(const cb_dev& d, const std::vector<cb_site>& sites, std::vector<st
 
 }  // namespace
 
-bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why) {
+bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why, double* rounds) {
+    if (rounds) *rounds = 0;
     auto no = [&](const std::string& w) {
         if (why) *why = w;
         return false;
@@ -283,6 +284,7 @@ bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* 
                       " B of shared memory each cannot be resident (" + std::string(cudaGetErrorString(e)) + ", " +
                       std::to_string(clusters) + " clusters)");
         }
+        if (rounds) *rounds += (double)classes[k].size() / clusters;
         if (k == 0) {
             if (threads) *threads = thr;
             if (smem) *smem = (size_t)a.smem_bytes;
