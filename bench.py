@@ -160,9 +160,9 @@ class Clocks:
 # bench step on 512 sites of the config-2 workload, per site (FP32): each launch loads
 # and stores every site once, so the traffic scales with the sites, not with the steps
 RESIDENT_DRAM_BYTES_PER_SITE = 319.7e6 / 512
-# ncu DRAM bytes (read + write) of one k_rd_s launch per cleft node (fp32, config-2 sites):
-# 129.3 MB + 78.5 MB on the 10 352 496 cleft nodes of 512 sites of this workload
-STREAM_CLEFT_DRAM_BYTES_PER_NODE = (129.278464e6 + 78.518016e6) / 10352496
+# ncu DRAM bytes (read + write) of one k_rd_t launch per cleft node (fp32, config-2 sites):
+# 546.5 MB + 470.5 MB on the 43 169 415 cleft nodes of 2048 sites of this workload
+STREAM_CLEFT_DRAM_BYTES_PER_NODE = (546.507008e6 + 470.451200e6) / 43169415
 
 
 def measured_peak_hbm():
@@ -229,7 +229,7 @@ def dominant_kernel(args, sim, sites, bytes_step, peak):
             "step_achieved_gbs": bytes_step / (step_ms / 1e3) / 1e9,
             "note": "achieved = the kernel's algorithmic bytes per launch (each stored value of its field read and "
                     "written once per node-step) / its CUDA-event launch time; traffic = ncu DRAM bytes per launch "
-                    "(measured on 512 sites of this workload, scaled by cleft nodes)"}
+                    "(measured on 2048 sites of this workload, scaled by cleft nodes)"}
 
 
 def cpu_model():

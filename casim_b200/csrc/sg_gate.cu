@@ -9,7 +9,7 @@
 // exchange through shared memory), the mouth values sit in shared memory. 2048 sites of 20 RyRs,
 // 20 windows of 20 steps with start and readback (the network and the feature and mouth kernels in
 // it took a third of the gain): 5.87 ms with the pools and the jSR on lane 0 and the mouths read
-// from global memory, 3.00 ms so.
+// from global memory, 2.80 ms so (3.00 with the pool's divisions done one by one).
 #include "engine.h"
 #include "pools.cuh"
 #include "resident_kernel.cuh"

@@ -966,6 +966,8 @@ constexpr int CH_OWNER = 1, CH_RIM = 2;  // flags of a RyR beside its node: take
 // launch of its own took 18 us of a 64-site step and this kernel 21 us, most of it waiting; the
 // efflux indices took integer divisions, the deposits went through an index list, the RyRs'
 // nodes were fetched twice and the sums reduced twice.
+// 4096 dyads, FP32: 45 + 131 us in two launches, 127 us in this one, of which the mouth and rim
+// gathers (a sector per value of an x edge) take over half.
 template <typename R, int NI, int NP, bool RD3D, bool GATE>
 __global__ void __launch_bounds__(UP_THREADS, 4)
     k_update_s(const __grid_constant__ cb_model m, const __grid_constant__ gate_args ga, const __grid_constant__ dep_args dep, int NS, bool want,
