@@ -153,7 +153,7 @@ void build_device(casim_b200_sim* h, int precision) {
     std::vector<cb_site> sites(d.S);
     std::vector<int> ch_node, ch_owner;
     std::vector<cb_site_scalars> sc(d.S);
-    std::vector<int> rim_cnode, dep_ptr, dep_term, dep_pos, dep_nptr(1, 0);
+    std::vector<int> rim_cnode, dep_ptr, dep_term, dep_pos, dep_nptr(1, 0), term_cn, next;
     std::vector<int3> dep_node;
     long long nb = 0;
     int choff = 0, rimoff = 0, termoff = 0;
@@ -201,30 +201,31 @@ void build_device(casim_b200_sim* h, int precision) {
                 rim_cnode.push_back(cn % mc + cfg.m.cpx * (cn / mc));
             }
             rimoff += nrim;
-            // deposit lists: efflux terms grouped by receiving cytosol node, term order kept
-            std::vector<std::vector<int>> lists(mc * mc);
+            // deposit lists: efflux terms grouped by receiving cytosol node, term order kept; for the
+            // specialised Update also the place of each term in the grouped order and the receiving nodes
+            st.term_off = termoff;
+            const int acc = T;
+            term_cn.resize(T);
+            next.assign((size_t)mc * mc + 1, 0);
             for (int t = 0; t < T; ++t) {
                 int x0, y0, x1, y1, x2, y2, z;
                 cb_efflux_term(t, st.nx, st.ny, zmax, x0, y0, x1, y1, x2, y2, z);
-                int r = cb_rim_index(x0, y0, st.nx, st.ny);
-                const int cn = rim_cnode[st.rim_off + r];
-                lists[cn % cfg.m.cpx + mc * (cn / cfg.m.cpx)].push_back(t);
+                const int cn = rim_cnode[st.rim_off + cb_rim_index(x0, y0, st.nx, st.ny)];
+                term_cn[t] = cn % cfg.m.cpx + mc * (cn / cfg.m.cpx);
+                ++next[term_cn[t] + 1];
             }
-            st.term_off = termoff;
-            int acc = 0;
             for (int cn = 0; cn < mc * mc; ++cn) {
-                dep_ptr.push_back(acc);
-                for (int t : lists[cn]) dep_term.push_back(t);
-                acc += (int)lists[cn].size();
+                next[cn + 1] += next[cn];
+                if (next[cn + 1] > next[cn]) dep_node.push_back(make_int3(cn, next[cn], next[cn + 1]));
             }
-            dep_ptr.push_back(acc);
-            // the same lists for the specialised Update: the place of each term in the grouped order,
-            // and the receiving nodes
-            dep_pos.resize((size_t)termoff + acc);
-            const int* p = dep_ptr.data() + dep_ptr.size() - (size_t)(mc * mc + 1);
-            for (int k = 0; k < acc; ++k) dep_pos[(size_t)termoff + dep_term[(size_t)termoff + k]] = k;
-            for (int cn = 0; cn < mc * mc; ++cn)
-                if (p[cn + 1] > p[cn]) dep_node.push_back(make_int3(cn, p[cn], p[cn + 1]));
+            dep_ptr.insert(dep_ptr.end(), next.begin(), next.end());
+            dep_term.resize((size_t)termoff + T);
+            dep_pos.resize((size_t)termoff + T);
+            for (int t = 0; t < T; ++t) {
+                const int k = next[term_cn[t]]++;
+                dep_term[(size_t)termoff + k] = t;
+                dep_pos[(size_t)termoff + t] = k;
+            }
             d.st_max_dn = std::max(d.st_max_dn, (int)dep_node.size() - dep_nptr.back());
             dep_nptr.push_back((int)dep_node.size());
             termoff += acc;
