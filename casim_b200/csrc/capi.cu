@@ -322,9 +322,9 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
             // and 31 us). Below the L2's size the resident step grows with the rounds in which the
             // sites take the chip's clusters, about 8.5 us a round with the RD3D cytosol, while the
             // streaming step starts at its launches' 31 us and grows by 0.25 us a site: streaming
-            // from 4.5 rounds on (us resident / streaming, FP32: sides 40..120, 48 sites, 3.7 rounds
-            // 33.8 / 32.9, 64 sites, 5.1 rounds 42.6 / 34.9; sides 40..60, 3.9 rounds 36.4 / 38.5,
-            // 4.9 rounds 45.8 / 41.9; sides 100..120, 64 sites, 9.1 rounds 79.3 / 39.0; with Mg,
+            // from the fifth round on (us resident / streaming, FP32: sides 40..120, 50 sites, 3.9 rounds
+            // 33.7 / 34.9, 56 sites, 4.5 rounds 40.3 / 34.9; sides 40..60, 3.9 rounds 33.9 / 36.3,
+            // 4.2 rounds 41.3 / 36.2; sides 100..120, 64 sites, 9.1 rounds 79.3 / 39.0; with Mg,
             // sides 40..60, 256 sites, 17 rounds 167 / 82). With a pool cytosol small sites take
             // one or two blocks each and stay faster resident (1200 sites of sides 40..60, 11
             // rounds: 64 / 89).
@@ -336,7 +336,7 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
             ck(cudaGetDevice(&dev), "cudaGetDevice");
             ck(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev), "cudaDeviceGetAttribute");
             const bool large = state > (size_t)l2;
-            if ((rd3d || h->d.m.dim == 3) && (large || (rd3d && rounds >= 4.5)) && cb_plain_streaming(h->d)) {
+            if ((rd3d || h->d.m.dim == 3) && (large || (rd3d && rounds > 4)) && cb_plain_streaming(h->d)) {
                 h->path = CASIM_PATH_PLAIN;
                 h->streams_by_rounds = !large;
                 h->resident_why = "streaming: state of " + std::to_string(state >> 20) + " MiB " + (large ? "exceeds the " : "of the ") +

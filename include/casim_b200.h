@@ -54,7 +54,7 @@ typedef enum { CASIM_FP64 = 0, CASIM_FP32 = 1 } casim_precision;
  *           1 or 3 cleft layers at every site): there the resident kernel's per-step
  *           chain of phases is slower than streaming the state from HBM. Also PLAIN
  *           for batches with the 3D cytosol of that layout whose sites would take the
- *           chip's clusters in 4.5 rounds or more. Otherwise RESIDENT when every site fits, else PLAIN. casim_b200_path_note says
+ *           chip's clusters in more than 4 rounds. Otherwise RESIDENT when every site fits, else PLAIN. casim_b200_path_note says
  *           which rule chose. */
 typedef enum { CASIM_PATH_AUTO = 0, CASIM_PATH_PLAIN = 1, CASIM_PATH_RESIDENT = 2 } casim_path;
 
