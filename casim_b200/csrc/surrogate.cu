@@ -940,17 +940,20 @@ casim_status casim_b200_sg_set_params(casim_sg h, const float* host) { return pa
 
 casim_status casim_b200_sg_forward(casim_sg h, const float* x_dev, int batch, float* y_dev) {
     if (!h || !x_dev || !y_dev || batch <= 0 || batch % BM) return CASIM_EINVAL;
+    // The one launch reads x while other CTAs already write y: an output over the input goes through
+    // the handle's own buffer.
+    const uintptr_t xa = (uintptr_t)x_dev, ya = (uintptr_t)y_dev;
+    const bool overlap = xa < ya + (size_t)batch * h->n_out * 4 && ya < xa + (size_t)batch * h->n_in * 4;
     cudaError_t e = cudaSuccess;
-    if (one_launch(h)) {
+    if (one_launch(h) && !overlap) {
         e = infer(h, x_dev, batch, y_dev, h->n_out, h->n_out);
-        if (e == cudaSuccess) e = check_err(h);
-        return e == cudaSuccess ? CASIM_OK : fail(h, e == cudaErrorLaunchTimeout ? CASIM_ETIMEOUT : CASIM_ECUDA, cudaGetErrorString(e));
+    } else {
+        e = ensure_capacity(h, batch);
+        if (e == cudaSuccess) e = one_launch(h) ? infer(h, x_dev, batch, h->Y, h->out_pad, h->n_out) : forward(h, x_dev, batch, false);
+        if (e == cudaSuccess)
+            e = cudaMemcpy2DAsync(y_dev, (size_t)h->n_out * 4, h->Y, (size_t)h->out_pad * 4, (size_t)h->n_out * 4, batch,
+                                  cudaMemcpyDeviceToDevice, h->stream);
     }
-    e = ensure_capacity(h, batch);
-    if (e == cudaSuccess) e = forward(h, x_dev, batch, false);
-    if (e == cudaSuccess)
-        e = cudaMemcpy2DAsync(y_dev, (size_t)h->n_out * 4, h->Y, (size_t)h->out_pad * 4, (size_t)h->n_out * 4, batch,
-                              cudaMemcpyDeviceToDevice, h->stream);
     if (e == cudaSuccess) e = check_err(h);
     return e == cudaSuccess ? CASIM_OK : fail(h, e == cudaErrorLaunchTimeout ? CASIM_ETIMEOUT : CASIM_ECUDA, cudaGetErrorString(e));
 }

@@ -332,7 +332,7 @@ casim_status casim_b200_sg_num_params(casim_sg h, int64_t* n);
 /* FP32 parameters in the layout of casim_b200_sg_num_params (host memory). */
 casim_status casim_b200_sg_get_params(casim_sg h, float* host);
 casim_status casim_b200_sg_set_params(casim_sg h, const float* host);
-/* y = net(x). */
+/* y = net(x); y may lie over x. */
 casim_status casim_b200_sg_forward(casim_sg h, const float* x_dev, int batch, float* y_dev);
 /* Mean-square loss over the n_out outputs and the gradient of every parameter
  * (host memory, parameter layout); no update. */
