@@ -331,9 +331,10 @@ __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, 
             t += -log(cbrng::u01d_fold(g)) * theta;
             const double r = cbrng::u01d_fold(g) * total;
             cbrng::u01d_fold(g);  // MakeTransition(runif()): a two-state channel flips
-            // the first channel whose cumulative rate reaches the draw (none: channel 0)
+            // the first channel whose cumulative rate reaches the draw (none: channel 0, which is also
+            // what no share of an infinite total amounts to)
             int idx = 0;
-            for (int j0 = 0; j0 < n_ch; j0 += 32) {
+            for (int j0 = 0; j0 < n_ch && total < INFINITY; j0 += 32) {
                 const unsigned hit = __ballot_sync(0xffffffffu, j0 + lane < n_ch && cum[min(j0 + lane, n_ch - 1)] >= r);
                 if (hit) {
                     idx = j0 + __ffs(hit) - 1;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(32 * QSL_WARPS) k_qs_lane(cb_model m, int n_ch
         const double theta = 1 / total;
         t += -log(cbrng::u01d_fold(g)) * theta;
         const double r = cbrng::u01d_fold(g) * total;
-        // the first RyR whose cumulative rate reaches the draw (none: RyR 0)
+        // the first RyR whose cumulative rate reaches the draw (none, or an infinite total: RyR 0)
         int idx = 0;
         {
             int lo = 0, hi = n_ch;  // the cumulative rates do not decrease
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(32 * QSL_WARPS) k_qs_lane(cb_model m, int n_ch
                 if (cum[mid * 32 + lane] >= r) hi = mid;
                 else lo = mid + 1;
             }
-            idx = lo < n_ch ? lo : 0;
+            idx = lo < n_ch && total < INFINITY ? lo : 0;
         }
         cbrng::u01d_fold(g);  // MakeTransition(runif()): a two-state channel flips
         mask ^= 1u << idx;
