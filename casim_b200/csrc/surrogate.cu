@@ -190,9 +190,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(const __grid_constant__ gem
         const int cg = n0 + c0;  // global column
         const size_t o = (size_t)row * g.N + cg;
         if (g.mode == EPI_PLAIN) {
-            float4* c = (float4*)(g.C + (size_t)blockIdx.z * g.M * g.N + o);
-            c[0] = make_float4(v[0], v[1], v[2], v[3]);
-            c[1] = make_float4(v[4], v[5], v[6], v[7]);
+            float* c = g.C + (size_t)blockIdx.z * g.M * g.N + o;
+            if (((uintptr_t)g.C & 15) == 0) {
+                ((float4*)c)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                ((float4*)c)[1] = make_float4(v[4], v[5], v[6], v[7]);
+            } else {  // a caller's output that begins anywhere
+#pragma unroll
+                for (int j = 0; j < 8; ++j) c[j] = v[j];
+            }
         } else if (g.mode == EPI_OUT) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) g.C[o + j] = v[j] + g.bias[cg + j];
@@ -1013,6 +1018,8 @@ casim_status casim_b200_sg_last_error(casim_sg h, char* buf, size_t n) {
 // for checking the kernel on its own: A [M][K], B [N][K] BF16 bit patterns.
 casim_status casim_b200_sg_gemm(const void* a_dev, const void* b_dev, int M, int N, int K, float* c_dev) {
     if (!a_dev || !b_dev || !c_dev) return CASIM_EINVAL;
+    // the operands arrive by 16-byte copies, the result leaves as floats
+    if (((uintptr_t)a_dev | (uintptr_t)b_dev) & 15 || (uintptr_t)c_dev & 3) return CASIM_EINVAL;
     casim_surrogate_s tmp;
     tmp.err_host = cb_take_flag();
     if (!tmp.err_host) return CASIM_ENOMEM;

@@ -385,7 +385,8 @@ casim_status casim_b200_sg_hybrid_run(casim_h h, casim_sg net, int32_t max_chann
                                       double ca_ref, casim_sg_hybrid_stats* stats);
 /* One product C = A . B^T on the tensor cores: A [M][K] and B [N][K] BF16
  * (bit patterns), C [M][N] FP32, all device memory; M a multiple of 128,
- * N a multiple of 16 in [16, 256], K a multiple of 64. */
+ * N a multiple of 16 in [16, 256], K a multiple of 64; A and B on 16-byte
+ * boundaries, C on any float (EINVAL otherwise). */
 casim_status casim_b200_sg_gemm(const void* a_dev, const void* b_dev, int M, int N, int K, float* c_dev);
 
 #ifdef __cplusplus
