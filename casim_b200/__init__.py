@@ -47,7 +47,7 @@ EXPORTS = (
     "casim_b200_sg_get_params", "casim_b200_sg_set_params", "casim_b200_sg_forward", "casim_b200_sg_gradients",
     "casim_b200_sg_train_step", "casim_b200_sg_check", "casim_b200_sg_launches", "casim_b200_sg_last_error",
     "casim_b200_sg_gemm", "casim_b200_trace_enable", "casim_b200_trace_count", "casim_b200_get_open_traces",
-    "casim_b200_release_analysis", "casim_b200_get_micro_states", "casim_b200_sg_hybrid_run", "casim_b200_autotune",
+    "casim_b200_release_analysis", "casim_b200_get_micro_states", "casim_b200_debug_give_up", "casim_b200_sg_hybrid_run", "casim_b200_autotune",
 )
 
 
@@ -147,6 +147,7 @@ def lib():
         L.casim_b200_last_step_launches.argtypes = [vp, ctypes.POINTER(ctypes.c_int64)]
         L.casim_b200_profile_step.argtypes = [vp, dp, i32, ip]
         L.casim_b200_set_site_gating.argtypes = [vp, ctypes.c_char_p, ctypes.c_char_p, ip, i32]
+        L.casim_b200_debug_give_up.argtypes = [vp]
         L.casim_b200_debug_rng.argtypes = [ctypes.POINTER(ctypes.c_uint32), i64, dp]
         L.casim_b200_set_site_jsr.argtypes = [vp, dp]
         L.casim_b200_path_note.argtypes = [vp, ctypes.c_char_p, ctypes.c_size_t]

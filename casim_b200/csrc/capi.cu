@@ -85,6 +85,11 @@ struct unsupported : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
+// a kernel's bounded wait ran out in an earlier launch: the state is not valid (CASIM_ETIMEOUT)
+struct gave_up : std::runtime_error {
+    gave_up() : std::runtime_error("a kernel's wait for its copies gave up: the state is not valid until the next start or reset") {}
+};
+
 template <typename T>
 T* dalloc(casim_b200_sim* h, size_t n) {
     void* p = nullptr;
@@ -119,15 +124,24 @@ casim_status set_err(casim_b200_sim* h, casim_status s, const std::string& msg) 
     catch (const unsupported& e) {                                          \
         return set_err(h, CASIM_EUNSUPPORTED, e.what());                    \
     }                                                                       \
+    catch (const gave_up& e) {                                              \
+        return set_err(h, CASIM_ETIMEOUT, e.what());                        \
+    }                                                                       \
     catch (const std::exception& e) {                                       \
         return set_err(h, CASIM_EINVAL, e.what());                          \
     }
 
-// a kernel's bounded wait for its own copies ran out in an earlier launch (the state is not valid)
-bool wait_gave_up(casim_b200_sim* h) {
-    if (!h->d.err_host || !*(volatile int*)h->d.err_host) return false;
-    h->err = "a kernel's wait for its copies gave up";
-    return true;
+// Waits for the handle's stream; every call that reads the state comes through here, so that none
+// returns a state that a kernel gave up on. Kernels set the error word in host memory; a reset
+// clears it in stream order.
+void drain(casim_b200_sim* h) {
+    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    if (*(volatile int*)h->d.err_host) throw gave_up();
+}
+// for calls that only queue work on the state: refused where it is known to be invalid (and no reset
+// is on its way)
+void refuse_invalid(casim_b200_sim* h) {
+    if (*(volatile int*)h->d.err_host) drain(h);
 }
 
 void check_site(casim_b200_sim* h, int site) {
@@ -511,7 +525,7 @@ casim_status casim_b200_set_site_jsr(casim_h h, const double* jsr) {
 casim_status casim_b200_step(casim_h h, int64_t n) {
     GUARD(h)
     if (n < 0) throw std::runtime_error("negative step count");
-    if (wait_gave_up(h)) return CASIM_ETIMEOUT;
+    refuse_invalid(h);
     long long launches = 0;
     ck(cudaEventRecord(h->ev0, h->stream), "cudaEventRecord");
     auto run = [&](long long k) {
@@ -547,7 +561,7 @@ casim_status casim_b200_profile_step(casim_h h, double* ms, int32_t n, int32_t* 
     GUARD(h)
     if (!ms || n < 1 || !count) throw std::runtime_error("profile_step: bad argument");
     if (h->tr) throw std::runtime_error("profile_step: not with an open-RyR trace enabled");
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     if (h->path == CASIM_PATH_RESIDENT) {
         long long launches = 0;
         ck(cudaEventRecord(h->ev0, h->stream), "cudaEventRecord");
@@ -571,6 +585,7 @@ casim_status casim_b200_profile_step(casim_h h, double* ms, int32_t n, int32_t* 
         *count = n < 4 ? n : 4;
     }
     h->timed = false;
+    drain(h);
     return CASIM_OK;
     END_GUARD(h)
 }
@@ -641,6 +656,7 @@ casim_status casim_b200_set_site_gating(casim_h h, const char* json_text, const 
 
 casim_status casim_b200_trace_enable(casim_h h, int64_t every_steps, int64_t max_samples) {
     GUARD(h)
+    refuse_invalid(h);  // sample 0 is the current state
     if (every_steps < 1 || max_samples < 1) throw std::runtime_error("trace needs every_steps >= 1 and max_samples >= 1");
     if ((double)max_samples * h->d.S * sizeof(uint16_t) > 16e9) throw std::runtime_error("trace larger than 16 GB");
     if (h->tr) {
@@ -670,7 +686,7 @@ casim_status casim_b200_get_open_traces(casim_h h, uint16_t* out) {
     GUARD(h)
     if (!out) throw std::runtime_error("null output");
     if (!h->tr) throw std::runtime_error("no trace: call casim_b200_trace_enable first");
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     ck(cudaMemcpy2D(out, (size_t)h->tr_n * sizeof(uint16_t), h->tr, (size_t)h->tr_max * sizeof(uint16_t),
                     (size_t)h->tr_n * sizeof(uint16_t), (size_t)h->d.S, cudaMemcpyDeviceToHost),
        "cudaMemcpy2D");
@@ -685,6 +701,7 @@ casim_status casim_b200_release_analysis(casim_h h, double hist_dt_ms, double ma
     if (!h->tr || h->tr_n < 1) throw std::runtime_error("no trace: call casim_b200_trace_enable first");
     if (!(hist_dt_ms > 0) || !(max_time_ms >= 0) || nadir < 0) throw std::runtime_error("bad histogram arguments");
     if (!per_site || !hist_all || !hist_quark || !hist_blip || !hist_spark || !class_counts) throw std::runtime_error("null output");
+    drain(h);
     const double ts = (double)h->tr_every * h->d.m.dt;  // ms between samples
     const long long nh = (long long)(max_time_ms / hist_dt_ms);  // CaSim/IndChannelCREAnalyzer.cpp:58
     if (nh > 100000000LL) throw std::runtime_error("histogram longer than 1e8 bins");
@@ -734,8 +751,7 @@ casim_status casim_b200_autotune(casim_h h, int64_t steps_per_trial, char* repor
 
 casim_status casim_b200_synchronize(casim_h h) {
     GUARD(h)
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
-    if (wait_gave_up(h)) return CASIM_ETIMEOUT;
+    drain(h);
     float ms = 0;
     // only after a step recorded both events; a failed query must not leave
     // its error behind for the next cudaGetLastError of another library
@@ -772,7 +788,7 @@ casim_status casim_b200_get_field(casim_h h, int32_t site, int32_t species, doub
     check_site(h, site);
     const cb_model& m = h->d.m;
     if (species < 0 || species >= m.F + m.n_buf) throw std::runtime_error("species out of range");
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     cb_site st;
     ck(cudaMemcpy(&st, h->d.sites + site, sizeof(cb_site), cudaMemcpyDeviceToHost), "cudaMemcpy");
     std::vector<double> blk((size_t)m.F * st.npad);
@@ -827,7 +843,7 @@ casim_status casim_b200_set_field(casim_h h, int32_t site, int32_t species, cons
 
 static casim_status get_scalars(casim_h h, int32_t site, cb_site_scalars& q) {
     check_site(h, site);
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     ck(cudaMemcpy(&q, h->d.sc + site, sizeof(cb_site_scalars), cudaMemcpyDeviceToHost), "cudaMemcpy");
     return CASIM_OK;
 }
@@ -836,7 +852,7 @@ casim_status casim_b200_get_mouth(casim_h h, int32_t site, int32_t species, doub
     GUARD(h)
     check_site(h, site);
     if (species < 0 || species >= h->d.NS) throw std::runtime_error("species out of range");
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     const cb_site_host& sh = h->cfg.sites[site];
     int nch = (int)sh.ch_node_xyz.size() / 3;
     cb_site st;
@@ -851,7 +867,7 @@ casim_status casim_b200_get_mouth(casim_h h, int32_t site, int32_t species, doub
 casim_status casim_b200_get_states(casim_h h, int32_t site, int32_t* out) {
     GUARD(h)
     check_site(h, site);
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     cb_site st;
     ck(cudaMemcpy(&st, h->d.sites + site, sizeof(cb_site), cudaMemcpyDeviceToHost), "cudaMemcpy");
     ck(cudaMemcpy(out, h->d.ch_state + st.ch_off, sizeof(int) * st.n_ch, cudaMemcpyDeviceToHost), "cudaMemcpy");
@@ -864,7 +880,7 @@ casim_status casim_b200_get_micro_states(casim_h h, int32_t site, int32_t* out) 
     check_site(h, site);
     if (!out) throw std::runtime_error("null output");
     if (!h->d.ch_micro) throw std::runtime_error("the RyR model has no micro-states (two-state gating)");
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     cb_site st;
     ck(cudaMemcpy(&st, h->d.sites + site, sizeof(st), cudaMemcpyDeviceToHost), "cudaMemcpy");
     ck(cudaMemcpy(out, h->d.ch_micro + st.ch_off, sizeof(int) * st.n_ch, cudaMemcpyDeviceToHost), "cudaMemcpy");
@@ -966,7 +982,7 @@ void sg_windows(casim_h h, casim_sg net, int max_channels, long long n, int wind
 }
 
 casim_status sg_net_status(casim_h h, casim_sg net) {
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     const cudaError_t en = cb_sg_net_error(net);
     if (en == cudaErrorLaunchTimeout) {
         h->err = "a tensor-core wait of the surrogate network gave up";
@@ -1056,7 +1072,7 @@ casim_status casim_b200_set_all_states(casim_h h, const int32_t* states) {
 
 casim_status casim_b200_get_all_states(casim_h h, int32_t* out) {
     GUARD(h)
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     ck(cudaMemcpy(out, h->d.ch_state, sizeof(int) * (size_t)h->d.total_ch, cudaMemcpyDeviceToHost), "cudaMemcpy");
     return CASIM_OK;
     END_GUARD(h)
@@ -1070,7 +1086,7 @@ casim_status casim_b200_get_all_mouth(casim_h h, int32_t species, double* out) {
     if (h->d.total_ch > 0) {
         if (!h->d.gathered) h->d.gathered = dalloc<double>(h, (size_t)h->d.total_ch);
         ck(cb_gather_mouth(h->d, species, h->d.gathered, h->stream), "gather mouth");
-        ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+        drain(h);
         ck(cudaMemcpy(out, h->d.gathered, (size_t)h->d.total_ch * sizeof(double), cudaMemcpyDeviceToHost), "cudaMemcpy");
     }
     return CASIM_OK;
@@ -1119,7 +1135,7 @@ casim_status casim_b200_get_cyto_field(casim_h h, int32_t site, int32_t species,
     check_site(h, site);
     if (h->d.m.cyto_type != CB_CYTO_RD3D) throw std::runtime_error("the cytosol is not RD3D");
     if (species < 0 || species >= h->d.CS) throw std::runtime_error("species out of range");
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     size_t rs = h->d.precision == 0 ? 8 : 4;
     std::vector<char> raw((size_t)h->d.nc * rs);
     const char* base = (const char*)h->d.cyto[h->d.ccur] + ((size_t)site * h->d.CS + species) * h->d.nc * rs;
@@ -1177,7 +1193,7 @@ casim_status casim_b200_get_release(casim_h h, int32_t site, double* out) {
 casim_status casim_b200_check_finite(casim_h h, int32_t* bad_site) {
     GUARD(h)
     if (bad_site) *bad_site = -1;
-    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    drain(h);
     const cb_model& m = h->d.m;
     size_t rs = h->d.precision == 0 ? 8 : 4;
     std::vector<cb_site> st(h->d.S);
@@ -1224,6 +1240,14 @@ __global__ void k_debug_rng(cbrng::State g, long long n, double* out) {
         for (long long k = 0; k < n; ++k) out[k] = cbrng::u01d(g);
 }
 }  // namespace
+
+extern "C" casim_status casim_b200_debug_give_up(casim_h h) {
+    GUARD(h)
+    ck(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    *(volatile int*)h->d.err_host = 1;
+    return CASIM_OK;
+    END_GUARD(h)
+}
 
 extern "C" casim_status casim_b200_debug_rng(const uint32_t seed[6], int64_t n, double* out) {
     if (!seed || !out || n < 0) return set_err(nullptr, CASIM_EINVAL, "bad argument");

@@ -29,8 +29,9 @@ namespace {
 
 template <typename R>
 __global__ void k_reset(cb_model m, const cb_site* __restrict__ sites, R* __restrict__ A, R* __restrict__ B,
-                        R* __restrict__ cur, cb_site_scalars* __restrict__ sc, int* __restrict__ ch_state) {
+                        R* __restrict__ cur, cb_site_scalars* __restrict__ sc, int* __restrict__ ch_state, int* __restrict__ err) {
     const int s = blockIdx.y;
+    if (s == 0 && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;  // the state is valid again
     const cb_site st = sites[s];
     const int F = m.F;
     R* a = A + st.node_base * F;
@@ -923,7 +924,7 @@ __global__ void k_sg_steps(cb_model m, int S, int NS, long long n, const cb_site
 template <typename R>
 cudaError_t reset_impl(cb_dev& d, cudaStream_t st) {
     dim3 g(std::max(1, std::min(64, (d.max_nodes + 255) / 256)), d.S);
-    k_reset<R><<<g, 256, 0, st>>>(d.m, d.sites, (R*)d.fields[0], (R*)d.fields[1], (R*)d.curgrid, d.sc, d.ch_state);
+    k_reset<R><<<g, 256, 0, st>>>(d.m, d.sites, (R*)d.fields[0], (R*)d.fields[1], (R*)d.curgrid, d.sc, d.ch_state, d.err_flag);
     d.cur = 0;
     if (d.m.cyto_type == CB_CYTO_RD3D) {
         dim3 gc((d.nc + 255) / 256, d.S);

@@ -36,7 +36,8 @@ typedef enum {
     CASIM_ECUDA = 2,       /* a CUDA runtime call failed (message carries cudaGetErrorString) */
     CASIM_ENOMEM = 3,      /* device allocation failed */
     CASIM_EUNSTABLE = 4,   /* explicit scheme violates dt*sum(2D/h^2) <= 1 for some species */
-    CASIM_ETIMEOUT = 5,    /* a bounded device wait gave up */
+    CASIM_ETIMEOUT = 5,    /* a bounded device wait gave up; a batch's state is then not valid, and calls that read
+                              it keep returning this, until its next reset or start */
     CASIM_ENONFINITE = 6,  /* a NaN/Inf was found in the state by casim_b200_check_finite */
     CASIM_EUNSUPPORTED = 7 /* configuration outside this build's limits */
 } casim_status;
@@ -255,6 +256,10 @@ casim_status casim_b200_set_site_gating(casim_h h, const char* json_text, const 
  * while an open-RyR trace is enabled. */
 casim_status casim_b200_profile_step(casim_h h, double* ms, int32_t n, int32_t* count);
 
+/* Diagnostic: leaves the batch as a kernel whose bounded wait ran out leaves it (every
+ * call that reads the state returns CASIM_ETIMEOUT until the next reset or start), for
+ * tests of a program's error handling. */
+casim_status casim_b200_debug_give_up(casim_h h);
 /* Diagnostic: n runif() draws of the MRG32k3a stream with the given seed,
  * generated by a device kernel (the generator every site's gating uses).
  * Reproduces RngStream::RandU01 with incPrec = true (CaSim/rngstream.cpp:271-283).
