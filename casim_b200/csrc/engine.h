@@ -61,6 +61,7 @@ struct cb_dev {
     void* st_runs = nullptr;  // the tiles of the asynchronous cleft kernel (stream::rd_tile), if it serves the batch
     int st_nruns = 0, st_grid = 0;
     bool st_cyt_ready = false;  // the asynchronous cytosol kernel's attributes are set
+    bool up_smem_set[2] = {false, false};  // the Update kernels' (without and with the gating)
     int st_stage[32];         // its shared-memory carve (stream::rd_stage)
     int st_nz = -1;
     unsigned* st_chcol = nullptr;  // bit per cleft column (node_base + x + px*y): holds a RyR

@@ -412,6 +412,18 @@ __global__ void __launch_bounds__(256) k_update(cb_model m, int NS, const cb_sit
         }
 }
 
+// A kernel's cap on dynamic shared memory is common to all handles, whose needs differ: always the
+// most a block can have, so that no handle (nor another thread) lowers it between this and a launch.
+cudaError_t allow_most_smem(const void* kern) {
+    cudaFuncAttributes fa;
+    int dev = 0, most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+}
+
 // jump table of the warp-parallel gating: row l < 32 holds A^(2l), both components, stored
 // entry-major (row 31, A^62, also takes a lane from one chunk of 32 draws to the next)
 bool pre_jump(cb_dev& d) {
@@ -588,9 +600,10 @@ cudaError_t launch_update_s(cb_dev& d, cudaStream_t st, bool gate, bool want) {
     size_t smem = (size_t)(d.max_ch + 7) / 8 * 8;
     if (RD3D) smem += (size_t)d.max_terms * dep.n * sizeof(double) + (size_t)dep.max_nodes * sizeof(int3);
     auto kern = gate ? stream::k_update_s<R, NI, NP, RD3D, true> : stream::k_update_s<R, NI, NP, RD3D, false>;
-    if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 40 * 1024 && !d.up_smem_set[gate]) {
+        const cudaError_t e = allow_most_smem((const void*)kern);
         if (e != cudaSuccess) return e;
+        d.up_smem_set[gate] = true;
     }
     // the rim reads the cytosol as it was before its latest step (RD3D coupling)
     kern<<<d.S, stream::UP_THREADS, smem, st>>>(d.m, gating(d), dep, d.NS, want, d.sites, (R*)d.fields[d.cur], (const R*)d.fields[1 - d.cur],
@@ -620,9 +633,10 @@ cudaError_t launch_update(cb_dev& d, cudaStream_t st, bool gate = false, bool wa
     }
     size_t smem = 256 * sizeof(double);
     if (d.m.cyto_type == CB_CYTO_RD3D) smem += (size_t)d.max_terms * d.m.F * sizeof(double);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_update<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && !d.up_smem_set[0]) {
+        const cudaError_t e = allow_most_smem((const void*)k_update<R>);
         if (e != cudaSuccess) return e;
+        d.up_smem_set[0] = true;
     }
     // the rim reads the cytosol as it was before its latest step (RD3D coupling)
     k_update<R><<<d.S, 256, smem, st>>>(d.m, d.NS, d.sites, (R*)d.fields[d.cur], (R*)d.curgrid, d.ch_node, d.ch_owner,
@@ -712,8 +726,7 @@ cudaError_t launch_rd_s(cb_dev& d, cudaStream_t st) {
         auto kern = d.st_nz == 1 ? stream::k_rd_t<R, NI, NP, 1, V, stream::RDT_STAGES> : stream::k_rd_t<R, NI, NP, 3, V, stream::RDT_STAGES>;
         cudaError_t e;
         if (d.st_grid == 0) {
-            // the cap of a kernel is shared by all handles, whose carves differ: always the most
-            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024)) != cudaSuccess) return e;
+            if ((e = allow_most_smem((const void*)kern)) != cudaSuccess) return e;
             int dev = 0, sms = 0, per = 0;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;

@@ -180,7 +180,7 @@ bool plan(const cb_dev& d, const std::vector<cb_site>& sites, const std::vector<
     a.max_rim = maxrim;
     a.FD = FD;
     if (rd3d && (maxt > 65535 || mc2 + 1 > 65535)) return false;  // u16 deposit tables
-    return off <= (size_t)(227 * 1024 - 1024);
+    return off <= (size_t)RS_MOST_SMEM;
 }
 
 // warps 0 and 1 run gating and the pools; the rest run the stencils

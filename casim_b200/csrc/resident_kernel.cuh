@@ -99,6 +99,8 @@ __device__ __forceinline__ fastdiv make_fastdiv(unsigned d) {
 }
 __device__ __forceinline__ int fdiv(int n, fastdiv f) { return (int)((__umulhi((unsigned)n, f.m) + (unsigned)n) >> f.s); }
 
+constexpr int RS_MOST_SMEM = 226 * 1024;  // dynamic shared memory of a block; the kernel's own variables take under 1 KiB
+
 template <bool B>
 struct bconst {
     static constexpr bool value = B;
@@ -1132,7 +1134,9 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
 template <typename R, int NI, int NPM, int NZ, int C>
 cudaError_t launch_one(const rs_args& a, int threads, cudaStream_t st, int n_sites, int* dry, int known) {
     auto kern = k_resident<R, NI, NPM, NZ, C>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_bytes);
+    // the cap is common to all handles, whose plans differ: always the most, so that no other thread
+    // lowers it between this and the launch
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_MOST_SMEM);
     if (e != cudaSuccess) return e;
     if (C > 8) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
