@@ -775,8 +775,10 @@ cudaError_t launch_cyto_s(cb_dev& d, cudaStream_t st) {
         kern<<<dim3(d.S, chunks), stream::CY_THREADS + 32, smem, st>>>(cy_constants<R>(d), chunk, in, out, d.cin, d.err_flag);
         return cudaGetLastError();
     }
-    const int per = (d.m.mc * d.m.cpx / V + stream::CY_THREADS - 1) / stream::CY_THREADS;
-    stream::k_cyto_v<R, NI, NCP, V><<<dim3(d.S, per), stream::CY_THREADS, 0, st>>>(cy_constants<R>(d), in, out, d.cin);
+    // a layer of fewer groups takes one block of its own size
+    constexpr int W = stream::cyv_vec(sizeof(R)), most = stream::cyv_threads(sizeof(R), NI + NCP);
+    const int groups = d.m.mc * d.m.cpx / W, thr = std::min(most, (groups + 31) / 32 * 32);
+    stream::k_cyto_v<R, NI, NCP, W><<<dim3(d.S, (groups + thr - 1) / thr), thr, 0, st>>>(cy_constants<R>(d), in, out, d.cin);
     return cudaGetLastError();
 }
 

@@ -595,19 +595,31 @@ __device__ __forceinline__ void cyto_reactions(const cy_const<R>& k, const group
 constexpr int cyt_blocks(int w, int CS) { return w == 4 ? (CS <= 3 ? 3 : 2) : (CS <= 3 ? 2 : 1); }
 constexpr int CYT_STAGES = 4;
 constexpr int CY_THREADS = 352;  // 13 groups x 25 rows of the shipped grid in 11 warps
-constexpr int cy_min_blocks(int w, int CS) { return w == 4 ? (CS <= 3 ? 3 : 2) : (CS <= 3 ? 2 : 1); }
+
+// k_cyto_v: nodes per thread, the most threads of a block, blocks per SM asked of the compiler and
+// planes loaded ahead of the next. A column's planes have to fit the registers: pairs of FP64 nodes, or
+// five species and more, in blocks of 352 threads spilled up to 1100 bytes, and layers of a few nodes left
+// most of such a block idle. Us of that shape / a thread per node with no planes ahead / this one: FP64,
+// three species, 1024 sites of 9^3 40 / 17 / 15, of 30^3 556 / 366 / 384, 256 of 40^3 364 / 244 / 209, six
+// species, 256 of 30^3 577 / 241 / 247; FP32, 1024 of 9^3 17.1 / 13.3 / 13.3, six species, 256 of 30^3
+// 206 / 163 / 124 (but of 24^3, which 352 threads hold whole, 76 / 108 / 85).
+constexpr int cyv_vec(int w) { return w == 4 ? CB_CYTO_VEC : 1; }
+constexpr int cyv_threads(int w, int CS) { return w == 4 && CS <= 4 ? 352 : 128; }
+constexpr int cyv_blocks(int w, int CS) { return w == 4 ? (CS <= 3 ? 3 : CS <= 4 ? 2 : 4) : (CS <= 3 ? 6 : CS <= 4 ? 4 : 3); }
+__host__ __device__ constexpr int cyv_ahead(int w, int CS) { return w == 4 ? (CS <= 4 ? 2 : 1) : (CS <= 5 ? 2 : 1); }
 
 // RD3D cytosol step on any grid: a thread per group of V nodes of a layer (blockIdx.y: groups
-// [y * CY_THREADS, ..)), marching the mc - 1 updated planes (the top plane is the bath) with planes
-// k-1 .. k+1 of its own nodes in registers and planes k+2, k+3 loaded ahead; plane 0 mirrors and
+// [y * blockDim.x, ..)), marching the mc - 1 updated planes (the top plane is the bath) with planes
+// k-1 .. k+1 of its own nodes in registers and up to two more loaded ahead; plane 0 mirrors and
 // takes the efflux deposits. The bath columns copy themselves so that every memory sector is
 // written whole (a partly written sector is read back from memory when it leaves L2).
 template <typename R, int NI, int NCP, int V>
-__global__ void __launch_bounds__(CY_THREADS, cy_min_blocks(sizeof(R), NI + NCP))
+__global__ void __launch_bounds__(cyv_threads(sizeof(R), NI + NCP), cyv_blocks(sizeof(R), NI + NCP))
     k_cyto_v(const __grid_constant__ cy_const<R> k, const R* __restrict__ in, R* __restrict__ out, const double* __restrict__ cin) {
-    constexpr int CS = NI + NCP;
+    constexpr int CS = NI + NCP, AHEAD = cyv_ahead(sizeof(R), CS), ROT = AHEAD + 2;
+    constexpr bool KEEP = sizeof(R) == 8;  // FP64 stores past L2 took 2 to 4 % longer
     const int mc = k.mc, px = k.px, npl = k.nplane, nc = k.nc;
-    const int col = ((int)blockIdx.y * CY_THREADS + (int)threadIdx.x) * V;
+    const int col = ((int)blockIdx.y * (int)blockDim.x + (int)threadIdx.x) * V;
     if (col >= npl) return;
     const int s = blockIdx.x, j = col / px, i = col - j * px;
     const bool bath = j == 0 || j == mc - 1;  // a whole row of the bath
@@ -621,15 +633,15 @@ __global__ void __launch_bounds__(CY_THREADS, cy_min_blocks(sizeof(R), NI + NCP)
         cu[c] = load_group<V>(v);
         hi[c] = load_group<V>(v + npl);
         p2[c] = load_group<V>(v + min(2, mc - 1) * npl);
-        p3[c] = load_group<V>(v + min(3, mc - 1) * npl);
+        if (AHEAD > 1) p3[c] = load_group<V>(v + min(3, mc - 1) * npl);
         lo[c] = hi[c];
     }
-#pragma unroll 4
+#pragma unroll ROT
     for (int kp = 0; kp < mc - 1; ++kp) {
         const int n = kp * npl;
         if (bath) {
 #pragma unroll
-            for (int c = 0; c < CS; ++c) store_group(o + c * nc + n, cu[c]);
+            for (int c = 0; c < CS; ++c) store_group(o + c * nc + n, cu[c], KEEP);
         } else {
             group<R, V> evo[CS];
 #pragma unroll
@@ -653,7 +665,7 @@ __global__ void __launch_bounds__(CY_THREADS, cy_min_blocks(sizeof(R), NI + NCP)
 #pragma unroll
                 for (int e = 0; e < V; ++e)
                     if (edge && (i + e == 0 || i + e >= mc - 1)) w.v[e] = cu[c].v[e];
-                store_group(o + c * nc + n, w);
+                store_group(o + c * nc + n, w, KEEP);
             }
         }
 #pragma unroll
@@ -661,8 +673,9 @@ __global__ void __launch_bounds__(CY_THREADS, cy_min_blocks(sizeof(R), NI + NCP)
             lo[c] = cu[c];
             cu[c] = hi[c];
             hi[c] = p2[c];
-            p2[c] = p3[c];
-            if (kp + 4 < mc) p3[c] = load_group<V>(u + c * nc + n + 4 * npl);
+            if (AHEAD > 1) p2[c] = p3[c];
+            group<R, V>& far = AHEAD > 1 ? p3[c] : p2[c];
+            if (kp + 2 + AHEAD < mc) far = load_group<V>(u + c * nc + n + (2 + AHEAD) * npl);
         }
     }
 }
