@@ -765,8 +765,9 @@ cudaError_t launch_cyto_s(cb_dev& d, cudaStream_t st) {
         // more) so that a small batch fills the chip; FP32, us for 1 / 2 / 3 / 4 chunks: 2048 sites
         // 148 / 154 / 166 / 177, 512 sites 51.5 / 45.9 / 47.3 / 47.4, 128 sites 19.2 / 16.6 / 15.2 / 15.4
         const int chunks = d.S >= 1024 ? 1 : d.S >= 256 ? 2 : 3, chunk = (planes + chunks - 1) / chunks;
-        constexpr int smem = stream::CYT_STAGES * (NI + NCP) * stream::cyt_planes<sizeof(R)>() * 25 * ((25 + V - 1) / V * V) * (int)sizeof(R);
-        auto kern = stream::k_cyto_t<R, NI, NCP, V, 25, stream::CYT_STAGES>;
+        constexpr int stages = stream::cyt_stages(sizeof(R), NI + NCP);
+        constexpr int smem = stages * (NI + NCP) * stream::cyt_planes<sizeof(R)>() * 25 * ((25 + V - 1) / V * V) * (int)sizeof(R);
+        auto kern = stream::k_cyto_t<R, NI, NCP, V, 25, stages>;
         if (!d.st_cyt_ready) {
             const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;

@@ -591,9 +591,11 @@ __device__ __forceinline__ void cyto_reactions(const cy_const<R>& k, const group
     }
 }
 
-// blocks of k_cyto_t per SM asked of the compiler, and stages a block keeps in flight
+// blocks of k_cyto_t per SM asked of the compiler, and stages a block keeps in flight: four, three
+// where four of six FP32 species would leave room for one block (2 ions, 4 pairs, 256 sites: 78 us with
+// four, 57 with three; a thread per node from global memory 68)
 constexpr int cyt_blocks(int w, int CS) { return w == 4 ? (CS <= 3 ? 3 : 2) : (CS <= 3 ? 2 : 1); }
-constexpr int CYT_STAGES = 4;
+__host__ __device__ constexpr int cyt_stages(int w, int CS) { return w == 4 && CS > 5 ? 3 : 4; }
 constexpr int CY_THREADS = 352;  // 13 groups x 25 rows of the shipped grid in 11 warps
 
 // k_cyto_v: nodes per thread, the most threads of a block, blocks per SM asked of the compiler and

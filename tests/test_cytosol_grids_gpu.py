@@ -47,3 +47,9 @@ def test_grid_matches_oracle(cuda_device, nodes, mg, extra, precision):
         for i, (a, b) in enumerate(pairs):
             assert (rel_err(a, b) <= 1e-11) if precision == "fp64" else (np.max(np.abs(a - b)) <= 1e-5 * np.max(np.abs(b))), (k, i)
     sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_shipped_grid_with_six_species(cuda_device, precision):
+    """25^3 with two ions and four pairs: as many species as the bulk copies' stages are counted for."""
+    test_grid_matches_oracle(cuda_device, 25, True, 2, precision)
