@@ -530,23 +530,9 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                 }
                 __syncwarp();
                 if (lane == 0) s_D = D;
-                // ---- jSR: coupling to the previous Update's currents, then its ODE
-                // (CaSim/SRPool.cpp:55-89) with the site's own beta
-                if (it > 0) {
-                    if (lane < NI) q.total[lane] = total_of(prv, lane);
-                    __syncwarp();
-                    if (lane == 0 && !m.jsr_const)
-                        for (int i = 0; i < NI; ++i) {
-                            q.IjSR[i] = q.total[i] * m.V_elem;
-                            q.nsr[i] = m.nsr[i];
-                            q.jsr[i] = q.jsr_new[i];
-                        }
-                }
-                if (lane == 0) cb_jsr_step<NI>(m, q, dt);
-                __syncwarp();
             } else if (warp == 1) {
                 // ---- cytosol pool: the previous Update's efflux, then its ODE
-                if (it > 0) {
+                if (it > 0 && !rd3d) {
                     for (int f = lane; f < F; f += 32) q.efflux[f] = efflux_of(prv, f);
                     __syncwarp();
                 }
@@ -598,6 +584,25 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                     }
                 }
                 asm volatile("bar.arrive 1, %0;" ::"r"(blockDim.x) : "memory");
+            }
+            if (warp == 0) {
+                // ---- jSR: coupling to the previous Update's currents, then its ODE
+                // (CaSim/SRPool.cpp:55-89) with the site's own beta. Only the Update needs it: with the
+                // RD3D cytosol it follows the deposits, which the worker warps wait for (FP32 us a step,
+                // the jSR before / after them: 50 dyads of 40 to 120 nodes a side 33.1 / 31.1, 500 sites of
+                // 12 to 24 nodes over 9^3 16.7 / 14.5; FP64, 100 of 40 to 60 over 16^3 31.8 / 29.9)
+                if (it > 0) {
+                    if (lane < NI) q.total[lane] = total_of(prv, lane);
+                    __syncwarp();
+                    if (lane == 0 && !m.jsr_const)
+                        for (int i = 0; i < NI; ++i) {
+                            q.IjSR[i] = q.total[i] * m.V_elem;
+                            q.nsr[i] = m.nsr[i];
+                            q.jsr[i] = q.jsr_new[i];
+                        }
+                }
+                if (lane == 0) cb_jsr_step<NI>(m, q, dt);
+                __syncwarp();
             }
             if (warp >= 2) {
                 // ---- worker warps: cleft stencil, strips of rows with a lane per x.
