@@ -281,16 +281,20 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
             const R* g = (const R*)a.fields + st.node_base * F;
             const int px = st.px;
             const fastdiv fd_nx = make_fastdiv(nx);
-            for (int f = 0; f < FP; ++f)
-                for (int z = 0; z < nz; ++z) {
-                    const R* src = g + (long long)f * np + (long long)px * (slo + (long long)ny * z);
-                    for (int k = tid; k < lstride; k += blockDim.x) {
-                        // stored rows have pitch px, rows in shared memory nx
-                        const R v = f < F ? src[k + fdiv(k, fd_nx) * (px - nx)] : (R)0;  // unused species slots hold zeros
-                        fa[f * cap + lstride * z + k] = v;
-                        fb[f * cap + lstride * z + k] = v;
+            // stored rows have pitch px, rows in shared memory nx; a node's place once for all species (one
+            // step of 1024 2D sites of 64 x 64 in a launch of its own: 263 us with a place per value, 235 so)
+            for (int z = 0; z < nz; ++z) {
+                const R* src = g + (long long)px * (slo + (long long)ny * z);
+                for (int k = tid; k < lstride; k += blockDim.x) {
+                    const int o = k + fdiv(k, fd_nx) * (px - nx), n = lstride * z + k;
+#pragma unroll
+                    for (int f = 0; f < FP; ++f) {
+                        const R v = f < F ? src[(long long)f * np + o] : (R)0;  // unused species slots hold zeros
+                        fa[f * cap + n] = v;
+                        fb[f * cap + n] = v;
                     }
                 }
+            }
             for (int k = tid; k < nloc; k += blockDim.x) chidx[k] = 0;
             const unsigned int* qs = (const unsigned int*)(a.sc + s);
             unsigned int* qd = (unsigned int*)&q;
@@ -298,14 +302,18 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
             for (int k = tid; k < NI; k += blockDim.x) ftab[k] = (R)0;
             if (rd3d) {
                 const R* cs = (const R*)a.cyto + (size_t)s * CS * nc;
-                for (int c = 0; c < CSM; ++c)
-                    for (int k = tid; k < cloc; k += blockDim.x) {
-                        const int row = k / mc;  // stored rows have pitch cpx, rows in shared memory mc
-                        const R v = c < CS ? cs[(size_t)c * nc + (size_t)(splo * mc + row) * m.cpx + (k - row * mc)] : (R)0;
-                        const int pl = k / mc2, l = pl * cps + (k - pl * mc2);
+                const fastdiv fd_mc = make_fastdiv(mc), fd_mc2 = make_fastdiv(mc2);
+                for (int k = tid; k < cloc; k += blockDim.x) {
+                    // stored rows have pitch cpx, rows in shared memory mc
+                    const int row = fdiv(k, fd_mc), o = (splo * mc + row) * m.cpx + (k - row * mc);
+                    const int pl = fdiv(k, fd_mc2), l = pl * cps + (k - pl * mc2);
+#pragma unroll
+                    for (int c = 0; c < CSM; ++c) {
+                        const R v = c < CS ? cs[(size_t)c * nc + o] : (R)0;
                         ca[c * ccap + l] = v;
                         cb[c * ccap + l] = v;
                     }
+                }
                 const int nrim = cb_rim_count(nx, ny);
                 for (int k = tid; k < nrim; k += blockDim.x) {
                     const int cn = a.rim_cnode[st.rim_off + k], jj = cn / m.cpx;
@@ -1092,12 +1100,16 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
             R* g = (R*)a.fields + st.node_base * F;
             const int px = a.sites[s].px;  // read again: not kept over the step loop
             const fastdiv fd_nx = make_fastdiv(nx);
-            for (int f = 0; f < F; ++f)
-                for (int z = 0; z < nz; ++z) {
-                    R* dst = g + (long long)f * np + (long long)px * (lo + (long long)ny * z);
-                    const R* src = fa + f * cap + lstride * z + nx * (lo - slo);
-                    for (int k = tid; k < nx * (hi - lo); k += blockDim.x) dst[k + fdiv(k, fd_nx) * (px - nx)] = src[k];
+            for (int z = 0; z < nz; ++z) {
+                R* dst = g + (long long)px * (lo + (long long)ny * z);
+                const R* src = fa + lstride * z + nx * (lo - slo);
+                for (int k = tid; k < nx * (hi - lo); k += blockDim.x) {
+                    const int o = k + fdiv(k, fd_nx) * (px - nx);
+#pragma unroll
+                    for (int f = 0; f < FP; ++f)
+                        if (f < F) dst[(long long)f * np + o] = src[f * cap + k];
                 }
+            }
             if (rank == 0) {
                 const unsigned int* qs = (const unsigned int*)&q;
                 unsigned int* qd = (unsigned int*)(a.sc + s);
@@ -1110,11 +1122,14 @@ __global__ void __launch_bounds__(max_threads(sizeof(R), NI + NPM, NZ, C), 1) k_
                     for (int j = 0; j < NI; ++j) cg_[(size_t)j * np + (cho[c] & ((1 << 30) - 1))] = ftab[(1 + c) * NI + j];
             if (rd3d) {
                 R* cd = (R*)a.cyto + (size_t)s * CS * nc;
-                for (int c = 0; c < CS; ++c)
-                    for (int k = tid; k < (phi - plo) * mc2; k += blockDim.x) {
-                        const int pl = k / mc2, row = k / mc;
-                        cd[(size_t)c * nc + (size_t)(plo * mc + row) * m.cpx + (k - row * mc)] = ca[c * ccap + (plo - splo + pl) * cps + (k - pl * mc2)];
-                    }
+                const fastdiv fd_mc = make_fastdiv(mc), fd_mc2 = make_fastdiv(mc2);
+                for (int k = tid; k < (phi - plo) * mc2; k += blockDim.x) {
+                    const int pl = fdiv(k, fd_mc2), row = fdiv(k, fd_mc);
+                    const int o = (plo * mc + row) * m.cpx + (k - row * mc), l = (plo - splo + pl) * cps + (k - pl * mc2);
+#pragma unroll
+                    for (int c = 0; c < CSM; ++c)
+                        if (c < CS) cd[(size_t)c * nc + o] = ca[c * ccap + l];
+                }
                 if (rank == r0 && a.nsteps > 0) {
                     // deposit of the final Update, for the next launch
                     const int pl = (int)((a.nsteps - 1) & 1);
