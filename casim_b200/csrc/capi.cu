@@ -322,7 +322,8 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
         size_t smem = 0;
         std::string why;
         double rounds = 0;
-        bool fits = cb_resident_fits(h->d, &thr, &smem, &why, &rounds);
+        int blocks = 0;
+        bool fits = cb_resident_fits(h->d, &thr, &smem, &why, &rounds, &blocks);
         h->resident_why = why;
         if (path == CASIM_PATH_RESIDENT && !fits) {
             std::string msg = "resident path unavailable: " + why;
@@ -333,15 +334,17 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
         if (path == CASIM_PATH_AUTO && fits) {
             // Large 3D batches stream faster than they run resident (4096 dyads with the RD3D
             // cytosol: 0.76 against 2.4 ms a step; 2D batches of 100 and 1024 sites: resident 4.4
-            // and 31 us). Below the L2's size the resident step grows with the rounds in which the
-            // sites take the chip's clusters, about 8.5 us a round with the RD3D cytosol, while the
-            // streaming step starts at its launches' 31 us and grows by 0.25 us a site: streaming
-            // from the fifth round on (us resident / streaming, FP32: sides 40..120, 50 sites, 3.9 rounds
-            // 33.7 / 34.9, 56 sites, 4.5 rounds 40.3 / 34.9; sides 40..60, 3.9 rounds 33.9 / 36.3,
-            // 4.2 rounds 41.3 / 36.2; sides 100..120, 64 sites, 9.1 rounds 79.3 / 39.0; with Mg,
-            // sides 40..60, 256 sites, 17 rounds 167 / 82). With a pool cytosol small sites take
-            // one or two blocks each and stay faster resident (1200 sites of sides 40..60, 11
-            // rounds: 64 / 89).
+            // and 28 us). Below the L2's size the resident step grows with the rounds in which the
+            // sites take the chip's clusters, the streaming step from its launches' 31 us with the
+            // sites' nodes. Sites of one or two blocks pack the chip so well that they stay resident
+            // (a pool cytosol, 1200 sites of sides 40..60, 11 rounds: us resident / streaming 64 / 89; RD3D, FP64,
+            // sides 12..24 over 9^3, 8 rounds 44 / 66; FP32 2D, sides 100..120 over 16^3, clusters of 2 and 4,
+            // 8 rounds 59 / 63). Sites of four and more stream from the fifth round on with
+            // the 25^3 cytosol (FP32, sides 40..60, 3.9 rounds 33.9 / 36.5, 4.3 rounds 45.9 / 37.0; sides 100..120,
+            // 4.3 rounds 42.0 / 33.0; 2D, 4.2 rounds 36.4 / 34.0; with Mg, 4.3 rounds 47.1 / 36.0; FP64 2D, 4.3
+            // rounds 41.6 / 32.2), from the seventh with other grids, whose streaming kernel is slower
+            // (FP64 2D over 16^3, 4.3 rounds 32.7 / 37.0, 6.3 rounds 45.7 / 43.0; FP32 with Mg over 9^3, 4.3 rounds
+            // 47.3 / 50.7, 6.3 rounds 66.3 / 65.3). A batch asked to take larger clusters stays resident.
             const bool rd3d = h->d.m.cyto_type == CB_CYTO_RD3D;
             const size_t w = precision == CASIM_FP64 ? 8 : 4;
             const size_t mc = (size_t)h->d.m.mc;
@@ -350,7 +353,8 @@ casim_status casim_b200_create(const char* json_text, const char* base_dir, casi
             ck(cudaGetDevice(&dev), "cudaGetDevice");
             ck(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev), "cudaDeviceGetAttribute");
             const bool large = state > (size_t)l2;
-            if ((rd3d || h->d.m.dim == 3) && (large || (rd3d && rounds > 4)) && cb_plain_streaming(h->d)) {
+            const bool many = rd3d && blocks >= 4 && h->d.min_cluster <= 1 && rounds > (h->d.m.mc == 25 ? 4 : 6);
+            if ((large ? rd3d || h->d.m.dim == 3 : many) && cb_plain_streaming(h->d)) {
                 h->path = CASIM_PATH_PLAIN;
                 h->streams_by_rounds = !large;
                 h->resident_why = "streaming: state of " + std::to_string(state >> 20) + " MiB " + (large ? "exceeds the " : "of the ") +

@@ -120,8 +120,9 @@ int* cb_take_flag();
 void cb_give_flag(int* f);
 
 // resident path (resident.cu)
-// rounds: how often the device's resident clusters are filled by the batch (fractions of the classes summed)
-bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why, double* rounds = nullptr);
+// rounds: how often the device's resident clusters are filled by the batch (fractions of the classes
+// summed); blocks: of the smallest cluster any site takes
+bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why, double* rounds = nullptr, int* blocks = nullptr);
 cudaError_t cb_resident_step(cb_dev& d, long long n, cudaStream_t st, long long* launches);
 // measured choice of block and cluster size per class (state unchanged); a description of
 // the choices into *report

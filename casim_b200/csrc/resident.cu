@@ -251,7 +251,7 @@ bool classify(const cb_dev& d, const std::vector<cb_site>& sites, std::vector<st
 
 }  // namespace
 
-bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why, double* rounds) {
+bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* why, double* rounds, int* blocks) {
     if (rounds) *rounds = 0;
     auto no = [&](const std::string& w) {
         if (why) *why = w;
@@ -288,6 +288,7 @@ bool cb_resident_fits(const cb_dev& d, int* threads, size_t* smem, std::string* 
         if (k == 0) {
             if (threads) *threads = thr;
             if (smem) *smem = (size_t)a.smem_bytes;
+            if (blocks) *blocks = cs[k];
         }
         if (why) {
             *why += (k ? ", " : "resident: ") + std::to_string(classes[k].size()) + " sites on clusters of " +

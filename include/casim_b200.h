@@ -54,9 +54,10 @@ typedef enum { CASIM_FP64 = 0, CASIM_FP32 = 1 } casim_precision;
  *           species layout the streaming kernels serve (1-2 ions, at most 4 pairs,
  *           1 or 3 cleft layers at every site): there the resident kernel's per-step
  *           chain of phases is slower than streaming the state from HBM. Also PLAIN
- *           for batches with the 3D cytosol of that layout whose sites would take the
- *           chip's clusters in more than 4 rounds. Otherwise RESIDENT when every site fits, else PLAIN. casim_b200_path_note says
- *           which rule chose. */
+ *           for batches with the 3D cytosol of that layout whose sites each take four
+ *           or more blocks and together the chip's clusters in more than 4 rounds (25^3
+ *           cytosol) or 6 (other grids). Otherwise RESIDENT when every site fits, else
+ *           PLAIN. casim_b200_path_note says which rule chose. */
 typedef enum { CASIM_PATH_AUTO = 0, CASIM_PATH_PLAIN = 1, CASIM_PATH_RESIDENT = 2 } casim_path;
 
 /* Optional per-site table (struct of arrays). Any NULL member falls back to
