@@ -18,27 +18,43 @@
 #include "physics.cuh"
 
 // Error words that kernels with bounded waits set, in mapped host memory so that a check costs no
-// copy. Page-locking takes milliseconds, so handles share pages of words: each takes a free one and
-// gives it back; a page is allocated when all words of the earlier ones are taken.
+// copy. Page-locking takes 1.8 ms, so handles share pages of words: each takes a free one and gives it
+// back; a page is allocated when all words of the earlier ones are taken. The list outlives every
+// static object (a handle may be destroyed from one), and a word whose page went with its context
+// (cudaDeviceReset) is dropped when it would be taken.
 namespace {
 std::mutex g_flag_lock;
-std::vector<int*> g_flags;
+std::vector<int*>& free_flags() {
+    static std::vector<int*>* const v = new std::vector<int*>;
+    return *v;
+}
+bool still_mapped(const int* f) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, f) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+}
 }  // namespace
-int* cb_take_flag() {
+int* cb_take_flag() try {
     std::lock_guard<std::mutex> g(g_flag_lock);
-    if (g_flags.empty()) {
+    std::vector<int*>& v = free_flags();
+    while (!v.empty() && !still_mapped(v.back())) v.pop_back();
+    if (v.empty()) {
         int* p = nullptr;
         if (cudaHostAlloc((void**)&p, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
-        for (int i = 0; i < 1024; ++i) g_flags.push_back(p + i);
+        for (int i = 0; i < 1024; ++i) v.push_back(p + i);
     }
-    int* f = g_flags.back();
-    g_flags.pop_back();
+    int* f = v.back();
+    v.pop_back();
     *f = 0;
     return f;
+} catch (const std::exception&) {
+    return nullptr;
 }
-void cb_give_flag(int* f) {
+void cb_give_flag(int* f) try {
     std::lock_guard<std::mutex> g(g_flag_lock);
-    g_flags.push_back(f);
+    free_flags().push_back(f);
+} catch (const std::exception&) {
 }
 
 struct casim_b200_sim {
