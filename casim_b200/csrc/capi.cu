@@ -197,7 +197,7 @@ void build_device(casim_b200_sim* h, int precision) {
         st.nz = cfg.m.dim == 3 ? sh.nz : 1;
         st.px = (st.nx + CB_CLEFT_VEC - 1) / CB_CLEFT_VEC * CB_CLEFT_VEC;
         int N = st.px * st.ny * st.nz;
-        st.npad = (N + 127) / 128 * 128;
+        st.npad = (N + CB_SITE_NODES - 1) / CB_SITE_NODES * CB_SITE_NODES;
         d.state_nodes += (st.nx * st.ny * st.nz + 31) / 32 * 32;
         st.node_base = nb;
         nb += st.npad;

@@ -97,6 +97,9 @@ struct cb_site_scalars {
 // Rows of the stored grids are padded to whole groups of nodes that a thread of the
 // streaming stencils loads and stores as one word (2 or 4 floats, 2 doubles).
 constexpr int CB_CLEFT_VEC = 4, CB_CYTO_VEC = 2;
+// Sites begin on multiples of this many nodes: 128 bits of the RyR bit map are the 16 bytes that a bulk
+// copy's source must be aligned to.
+constexpr int CB_SITE_NODES = 128;
 
 // Packed site table entry (device resident, read-only during stepping).
 // Fields of site s: species f, node n (x fastest: n = x + px*(y + ny*z), px = nx rounded up
@@ -105,7 +108,7 @@ constexpr int CB_CLEFT_VEC = 4, CB_CYTO_VEC = 2;
 struct cb_site {
     int nx, ny, nz, px;
     int n_ch;
-    int npad;              // px*ny*nz rounded up to a multiple of 32
+    int npad;              // px*ny*nz rounded up to whole CB_SITE_NODES nodes
     int ch_off;            // first RyR of the site in the channel arrays
     long long node_base;   // sum of npad over the preceding sites
     int rim_off;           // RD3D: first rim entry of the site (rim -> cytosol node table)

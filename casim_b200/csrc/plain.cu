@@ -468,6 +468,8 @@ int stream_tiles(cb_dev& d) {
     std::vector<int4> tiles;
     std::vector<stream::rd_tile> runs;
     const int tn = stream::rdt_threads(d.precision == 0 ? 8 : 4) * V;
+    static_assert(CB_SITE_NODES % 128 == 0 && stream::rdt_threads(4) * stream::rd_vec(4) % 128 == 0 && stream::rdt_threads(8) * stream::rd_vec(8) % 128 == 0,
+                  "a tile's RyR bits begin on 16 bytes");
     int px_min = INT32_MAX, px_max = 0;
     bool two_rims = false;  // a tile may hold a site's first and last row
     for (int s = 0; s < d.S; ++s) {
