@@ -487,7 +487,8 @@ class QuasiStationarySites:
     """Quasi-stationary release sites simulated with Gillespie's method on the device:
     the reference's ParallelSolver path (CaSim/ParallelSolver.cpp:51-143,
     CaSim/QuasyStationaryReleaseSite.cpp:89-133) with the mouth Ca of the linearised
-    Naraghi-Neher model (CaSim/LinearNaraghiNeher.cpp:9-75), one scenario per warp."""
+    Naraghi-Neher model (CaSim/LinearNaraghiNeher.cpp:9-75), one scenario per lane for sites of
+    up to 32 RyRs, per warp for larger ones."""
 
     def __init__(self, params, n_scenarios, base_dir=None, seeds=None, max_events=4096, json_text=None):
         L = lib()

@@ -1,5 +1,5 @@
-// Pool ODEs of one site, shared by the one-thread-per-site kernels of the
-// plain path and the surrogate-driven gating.
+// Pool ODEs of one site: the resident kernel, the Update of the streaming path, the generic kernels
+// and the surrogate-driven gating step them here.
 #pragma once
 #include "model.h"
 

@@ -246,7 +246,8 @@ struct qs_rate<CB_TWO_STATE_MWC> {
 
 constexpr int QS_WARPS = 4;  // warps per block
 
-// Shared memory of a block of k_qs_run: the increments where they fit (n_ch <= 64), then per warp
+// Shared memory of a block of k_qs_run: the increments of up to 64 RyRs (2048 scenarios of 64: 719 us, 741
+// from L1; of 72: 1119 and 1116, beside 48 KiB a block), then per warp
 // the cumulative rates and the open-channel bitmask, padded to 16 bytes so that every warp's
 // rates start 8-byte aligned.
 __host__ __device__ inline size_t qs_warp_bytes(int n_ch) {
@@ -255,8 +256,8 @@ __host__ __device__ inline size_t qs_warp_bytes(int n_ch) {
 __host__ __device__ inline size_t qs_added_bytes(int n_ch) { return n_ch <= 64 ? sizeof(double) * n_ch * n_ch : 0; }
 
 // Scenarios on persistent warps (CaSim/QuasyStationaryReleaseSite.cpp:89-133). 4096 scenarios of a
-// 48-RyR MWC site, run and analysis: 2.60 ms with lane 0 summing the rates and walking the shares,
-// 2.02 ms by scans over the lanes.
+// 48-RyR MWC site, the run's kernel: 2.33 ms with lane 0 summing the rates and walking the shares,
+// 1.77 ms by scans over the lanes.
 template <int MODEL>
 __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, const double* __restrict__ added, double bg, double mg,
                                                           double max_time, int n_scen, const int* __restrict__ first,
@@ -370,8 +371,8 @@ __global__ void __launch_bounds__(32 * QS_WARPS) k_qs_run(cb_model m, int n_ch, 
 // register; each event every running lane forms the mouth Ca of all RyRs (the increments
 // of the open RyRs in RyR order), the rates and their running sum (kept in shared memory, a
 // column per lane), the draws and the pick, for 32 scenarios at once. Lanes take the next
-// scenario off the counter when theirs ends. 131072 scenarios of a 20-RyR MWC site, run and
-// analysis: 11.8 ms with a select per increment, five divisions per rate and one per share, 7.0 ms.
+// scenario off the counter when theirs ends. 131072 scenarios of a 20-RyR MWC site,
+// the kernel alone: 9.5 ms with a select per increment, five divisions per rate and one per share, 5.0 ms.
 constexpr int QSL_WARPS = 4;
 __host__ __device__ inline size_t qsl_smem(int n_ch) {
     return sizeof(double) * ((size_t)n_ch * n_ch + (size_t)QSL_WARPS * 32 * n_ch);

@@ -972,7 +972,9 @@ constexpr int CH_OWNER = 1, CH_RIM = 2;  // flags of a RyR beside its node: take
 // One site per block. GATE (a time step): first the RyR gating (warp 0) and the pool ODEs (warp
 // 1), which nothing before them in the step needs, while the other warps form the efflux; then
 // the Update (CaSim/ParallelHybridSolver.cpp:159-175): mouth values, Dirichlet rim from the
-// cytosol (RD3D: k_rd_t set it), efflux through the rim, the RD3D deposits into cytosol layer 0,
+// cytosol (RD3D: k_rd_t set it), efflux through the rim, the RD3D deposits into cytosol layer 0 (each
+// receiving node's terms in a fixed order of eight interleaved partial sums, equal to their sum in term
+// order within rounding),
 // RyR currents, the jSR coupling and the probabilities of the next gating. Without GATE (the
 // public Update) no time passes and the rim is always set here. want: also write what only
 // the getters read (mouth values, RD3D: efflux sums), for the last step of a call.

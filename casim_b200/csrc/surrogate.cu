@@ -237,9 +237,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(const __grid_constant__ gem
 // the weights stream from L2 in K slices of 64, three stages ahead of the tensor core and across
 // the layer boundary, so that the next layer's first slices load during an epilogue. The products
 // run over the same K order into one TMEM accumulator, so the outputs equal the layer-by-layer
-// ones. 16384 rows of the 63 -> 4 x 256 -> 20 network through the public call: 194 us as a cast, five
-// products, a copy of the used columns and an error read-back, 71 us this way; what remains is the
-// GELU epilogues (erf on the FP32 pipe, about 4.5 us a layer) and the call's synchronisation.
+// ones. 16384 rows of the 63 -> 4 x 256 -> 20 network through the public call: 200 us as a cast, five
+// products, a copy of the used columns and an error read-back, 71 us this way, of which the kernel
+// takes about 60 (62 from a cold L2: issue slots 41 % busy, the tensor pipe 7 %): 8 warps wait for a
+// layer's products, then evaluate its GELUs (erf on the FP32 pipe) while the tensor core waits.
 constexpr int MLP_LAYERS = 16, MLP_THREADS = 256, MLP_STAGES = 3;
 constexpr int MLP_B_STAGE = 256 * BK * 2;  // 32 KiB
 constexpr int MLP_SMEM = 4 * A_STAGE + MLP_STAGES * MLP_B_STAGE;
@@ -627,12 +628,9 @@ cudaError_t ensure_capacity(casim_sg h, int B) {
     return cudaSuccess;
 }
 
-// inference: the whole network in one launch; y [B][ldy], ncols columns of it written
-bool one_launch(const casim_surrogate_s* h) {
-    bool ok = h->L <= MLP_LAYERS;
-    for (int l = 0; l < h->L; ++l) ok = ok && h->dout[l] % 32 == 0;
-    return ok;
-}
+// inference: the whole network in one launch (widths are multiples of 64, so an epilogue's column
+// halves are whole 16-column reads); y [B][ldy], ncols columns of it written
+bool one_launch(const casim_surrogate_s* h) { return h->L <= MLP_LAYERS; }
 cudaError_t infer(casim_sg h, const float* x, int B, float* y, int ldy, int ncols) {
     mlp_args g{};
     g.x = x;

@@ -284,7 +284,8 @@ casim_status casim_b200_rng_draws_static(const uint32_t seed[6], int64_t n, doub
 
 /* ---- Quasi-stationary release sites: the reference's ParallelSolver path
  * (CaSim/ParallelSolver.cpp:51-143, CaSim/QuasyStationaryReleaseSite.cpp:89-133)
- * batched on the device, one scenario per warp. The mouth Ca of every RyR is the
+ * batched on the device, one scenario per lane for sites of up to 32 RyRs, per warp
+ * for larger ones. The mouth Ca of every RyR is the
  * background plus the linearised Naraghi-Neher increments of the open RyRs
  * (CaSim/LinearNaraghiNeher.cpp:9-75, computed on the host); gating is simulated
  * exactly with Gillespie's method (total rate, exponential waiting time, channel
